@@ -24,13 +24,21 @@ cudaError_t attn_dense_tc5(void *out, const void *q, const void *k, const void *
                            unsigned batch, unsigned lq, unsigned lk, unsigned heads,
                            unsigned kv_heads, float scale, cudaStream_t stream,
                            const PeerOutput *peer = nullptr);
+// Causal attention of a sequence with itself (bf16, head dim 128, grouped-query), and fp16 with head
+// dim 64: the same kernel in two further instantiations.
+cudaError_t attn_causal_tc5(void *out, const void *q, const void *k, const void *v, float *lse, unsigned batch,
+                            unsigned sequence, unsigned heads, unsigned kv_heads, float scale, cudaStream_t stream);
+cudaError_t attn_f16_d64_tc5(void *out, const void *q, const void *k, const void *v, float *lse, unsigned batch,
+                             unsigned sequence, unsigned heads, float scale, cudaStream_t stream);
 // Two query tiles per CTA (attn_tc5_pair.cu); tensor maps as built by attn_dense_tc5.
+enum class PairKind { BF16_D128, BF16_D128_CAUSAL, F16_D64 };
 cudaError_t attn_dense_tc5_pair(const ::CUtensorMap_st *mq, const ::CUtensorMap_st *mk,
                                 const ::CUtensorMap_st *mv, void *out, float *lse, unsigned batch,
                                 unsigned lq, unsigned lk, unsigned heads, unsigned kv_heads,
                                 float scale, int *status, cudaStream_t stream,
                                 const PeerOutput *peer = nullptr, unsigned segments = 0,
-                                const unsigned *segment_rows = nullptr, unsigned split_tiles = 0);
+                                const unsigned *segment_rows = nullptr, unsigned split_tiles = 0,
+                                PairKind kind = PairKind::BF16_D128);
 // Split-KV (batch 1): with split_tiles > 0 the launch above cuts the keys into slices of
 // split_tiles 128-row tiles on grid.z and writes per-slice outputs [slices][lq][heads][128] bf16 and
 // logsumexp [slices][heads][lq] f32 (both required); this combines them.

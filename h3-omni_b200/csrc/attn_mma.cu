@@ -1,12 +1,8 @@
-// Warp-level (mma.sync m16n8k16) flash attention forward for the two link-completeness
-// variants that are off the DiT hot path:
-//   - bf16, head dim 128, causal and/or grouped-query (h3_flash_bf16; the reference's
-//     FlashAttention-2 adapter, cuda/flash_attention.cu:29-67, used by its text and vision
-//     encoders and by the FastH3 refiner), and
-//   - fp16, head dim 64, non-causal (h3_flash3_f16_d64, cuda/flash3_attention.cu:81-87,
-//     video VAE).
-// Sequences there are short, so this kernel aims at correctness and portability of shapes
-// (any Lq, Lk, batch, GQA ratio), not at tensor-core peak; the dense DiT path uses attn_tc5.cu.
+// Warp-level (mma.sync m16n8k16) flash attention forward for the causal / grouped-query bf16 call
+// (head dim 128, h3_flash_bf16; the reference's cuda/flash_attention.cu:29-67) and the fp16 call (head
+// dim 64, h3_flash3_f16_d64, cuda/flash3_attention.cu:81-87) when the query or the output does not
+// start on a 16-byte boundary. Aligned tensors go to attn_tc5_pair.cu, which needs the boundary (TMA
+// loads, 16-byte stores) and is 5 to 10 times as fast.
 //
 // A CTA of 4 warps owns 64 query rows (16 per warp) and walks KV tiles of 64 rows staged in
 // shared memory (K row-major, V transposed so both MMA B operands are 32-bit loads).

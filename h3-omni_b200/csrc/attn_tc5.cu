@@ -452,13 +452,13 @@ EncodeTiled encode_fn() {
     return fn;
 }
 
-// Rank-4 bf16 map with a 64-element (128-byte) swizzled inner box.
+// Rank-4 map of 16-bit floats with a 64-element (128-byte) swizzled inner box.
 cudaError_t make_map(CUtensorMap *map, const void *base, const uint64_t dims[4],
-                     const uint64_t strides_bytes[3], const uint32_t box[4]) {
+                     const uint64_t strides_bytes[3], const uint32_t box[4], bool f16 = false) {
     EncodeTiled fn = encode_fn();
     if (!fn) return cudaErrorNotSupported;
     const cuuint32_t ones[4] = {1, 1, 1, 1};
-    CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<void *>(base), dims,
+    CUresult r = fn(map, f16 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<void *>(base), dims,
                     strides_bytes, box, ones, CU_TENSOR_MAP_INTERLEAVE_NONE,
                     CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                     CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
@@ -554,6 +554,43 @@ cudaError_t attn_dense_tc5(void *out, const void *q, const void *k, const void *
                                    status, stream, peer);
     dim3 grid((lq + BM - 1) / BM, heads, batch);
     return launch<128, false>(mq, mk, mv, p, grid, stream);
+}
+
+namespace {
+// Token-major [batch][rows][heads][dim] tensor read in boxes of 128 rows x 64 elements.
+cudaError_t token_major_map(CUtensorMap *map, const void *base, unsigned dim, unsigned heads, unsigned rows,
+                            unsigned batch, bool f16) {
+    const uint64_t row = (uint64_t)heads * dim * 2;
+    const uint64_t dims[4] = {dim, heads, rows, batch}, strides[3] = {dim * 2, row, rows * row};
+    const uint32_t box[4] = {64, 1, 128, 1};
+    return make_map(map, base, dims, strides, box, f16);
+}
+cudaError_t self_attention_tc5(PairKind kind, unsigned dim, void *out, const void *q, const void *k, const void *v,
+                               float *lse, unsigned batch, unsigned sequence, unsigned heads, unsigned kv_heads,
+                               float scale, cudaStream_t stream) {
+    if (!batch || !sequence || !heads || !kv_heads || heads % kv_heads) return cudaErrorInvalidValue;
+    if (heads > 65535u || batch > 65535u) return cudaErrorInvalidValue;
+    const bool f16 = kind == PairKind::F16_D64;
+    int *status = nullptr;
+    cudaError_t e = device_status_word(&status);
+    CUtensorMap mq, mk, mv;
+    if (e == cudaSuccess) e = token_major_map(&mq, q, dim, heads, sequence, batch, f16);
+    if (e == cudaSuccess) e = token_major_map(&mk, k, dim, kv_heads, sequence, batch, f16);
+    if (e == cudaSuccess) e = token_major_map(&mv, v, dim, kv_heads, sequence, batch, f16);
+    if (e != cudaSuccess) return e;
+    return attn_dense_tc5_pair(&mq, &mk, &mv, out, lse, batch, sequence, sequence, heads, kv_heads, scale, status,
+                               stream, nullptr, 0, nullptr, 0, kind);
+}
+}  // namespace
+
+cudaError_t attn_causal_tc5(void *out, const void *q, const void *k, const void *v, float *lse, unsigned batch,
+                            unsigned sequence, unsigned heads, unsigned kv_heads, float scale, cudaStream_t stream) {
+    return self_attention_tc5(PairKind::BF16_D128_CAUSAL, 128, out, q, k, v, lse, batch, sequence, heads, kv_heads,
+                              scale, stream);
+}
+cudaError_t attn_f16_d64_tc5(void *out, const void *q, const void *k, const void *v, float *lse, unsigned batch,
+                             unsigned sequence, unsigned heads, float scale, cudaStream_t stream) {
+    return self_attention_tc5(PairKind::F16_D64, 64, out, q, k, v, lse, batch, sequence, heads, heads, scale, stream);
 }
 
 cudaError_t attn_segments_tc5(void *out, const void *q, const void *const *k, const void *const *v,

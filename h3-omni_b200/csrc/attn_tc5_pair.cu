@@ -1,4 +1,5 @@
-// Dense attention forward, two query tiles per CTA (tcgen05 + TMEM + TMA), bf16, head dim 128.
+// Dense attention forward, two query tiles per CTA (tcgen05 + TMEM + TMA): bf16 with head dim 128,
+// non-causal or causal, and fp16 with head dim 64.
 //
 // The single-tile kernel in attn_tc5.cu relies on two co-resident CTAs to overlap softmax
 // with MMAs, but nothing keeps the two CTAs out of phase, and each loads K/V for itself.
@@ -31,6 +32,8 @@
 // has more than one query tile (replacing the reference's cuda/flash3_attention.cu:18-94).
 #include <cuda.h>
 
+#include <type_traits>
+
 #include "attn_kernels.h"
 #include "softmax_tc5.cuh"
 
@@ -39,14 +42,24 @@ namespace {
 
 constexpr int PBM = 128, PBN = 128, PHD = 128;
 constexpr int PAIR_THREADS = 384;                  // three warpgroups: softmax A, softmax B, {TMA, MMA}
-constexpr int PAIR_STAGES = 5;                      // K0 V0 K1 V1 ... ring of 32 KB tiles
-constexpr int PAIR_TILE_BYTES = PBN * PHD * 2;      // 32 KB
-constexpr int PAIR_HALF_BYTES = PBN * 128;          // one 64-column half
-constexpr int PAIR_Q_BYTES = 2 * PBM * PHD * 2;     // 64 KB
-constexpr int PAIR_SMEM_BYTES = PAIR_Q_BYTES + PAIR_STAGES * PAIR_TILE_BYTES + 1024;
+constexpr int PAIR_SOFTMAX_REGS = 208, PAIR_OTHER_REGS = 88;   // what setmaxnreg leaves the warpgroups with
+constexpr int PAIR_HALF_BYTES = PBN * 128;          // one 64-column half of a tile
 constexpr int PAIR_O_COL = 256;
 constexpr float PAIR_RESCALE_LOG2 = 8.0f;
-constexpr int PAIR_POLY_EVERY = 0x55;               // which groups of four columns take a pair of exponentials on the FMA pipe (25 %)
+
+// What depends on the head dimension. HD = 128: 64 KB of Q and five slots of 32 KB. HD = 64: half
+// of each, so the ring gets eight slots; the products take half the time, the softmax the same, so
+// the exponential unit is the critical resource and half of the exponentials leave it.
+template <int HD>
+struct PairConfig {
+    static constexpr int STAGES = HD == 128 ? 5 : 8;      // K0 V0 K1 V1 ... ring of tiles
+    static constexpr int HALVES = HD / 64;
+    static constexpr int TILE_BYTES = PBN * HD * 2;
+    static constexpr int Q_TILE_BYTES = PBM * HD * 2;
+    static constexpr int SMEM_BYTES = 2 * Q_TILE_BYTES + STAGES * TILE_BYTES + 1024;
+    // which groups of four columns take a pair of exponentials on the FMA pipe (25 % / 50 %)
+    static constexpr int POLY = HD == 128 ? 0x55 : 0xff;
+};
 
 #ifdef H3B_TRACE
 // Development aid, compiled only with -DH3B_TRACE: cycle counters of CTA (0,0,0).
@@ -74,18 +87,23 @@ struct PairParams {
     // they were batch element blockIdx.z, and merge_splits_kernel combines the slices.
     int split_tiles;
     float scale, scale_log2;
-    __nv_bfloat16 *out;
+    uint16_t *out;   // bf16, or fp16 in the fp16 kernel
     float *lse;
     int *status;
     // sequence-gather fused into the epilogue (see PeerOutput); rows_per_rank == 0: off
-    __nv_bfloat16 *peer_out[16];
+    uint16_t *peer_out[16];
     unsigned rows_per_rank, rank, total_heads;
 };
 
+// CAUSAL: key k is attended by query rows >= k (lq == lk); every query tile walks its own number of
+// key tiles. Work is handed out longest walk first: blockIdx.x is the head, blockIdx.y counts the
+// pairs of query tiles from the end.
+template <int HD, bool F16, bool CAUSAL>
 __global__ void __launch_bounds__(PAIR_THREADS, 1)
 attn_tc5_pair_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ PairKvMaps kv,
                      const PairParams p) {
-    constexpr int ST = PAIR_STAGES;
+    using Cfg = PairConfig<HD>;
+    constexpr int ST = Cfg::STAGES;
     extern __shared__ uint8_t smem_raw[];
     __shared__ uint64_t bars[1 + 2 * ST + 9];
     __shared__ uint32_t tmem_slot;
@@ -95,7 +113,7 @@ attn_tc5_pair_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
     const uint32_t q_smem = smem_base;
-    const uint32_t ring = q_smem + PAIR_Q_BYTES;
+    const uint32_t ring = q_smem + 2 * Cfg::Q_TILE_BYTES;
 
     const uint32_t bar0 = smem_u32(bars);
     const uint32_t bar_q_full = bar0;
@@ -108,15 +126,21 @@ attn_tc5_pair_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
     auto bar_p_full = [&](int t, int piece) { return bar0 + 8u * (1 + 2 * ST + 2 + 3 * t + piece); };
     const uint32_t bar_pv_done = bar0 + 8u * (1 + 2 * ST + 8);   // the last PV of both tiles
 
-    const int head = blockIdx.y, batch = p.split_tiles ? 0 : blockIdx.z, out_batch = blockIdx.z;
+    const int head = CAUSAL ? blockIdx.x : blockIdx.y, batch = p.split_tiles ? 0 : blockIdx.z, out_batch = blockIdx.z;
     const int kv_head = head / (p.heads / p.kv_heads);
-    const int q_row0 = blockIdx.x * 2 * PBM;
+    const int q_row0 = (CAUSAL ? gridDim.y - 1 - blockIdx.y : blockIdx.x) * 2 * PBM;
     const int tile0 = p.split_tiles * (int)blockIdx.z;   // first key tile of this CTA's slice (0 without split)
     // key rows of range s as this CTA sees it (a split call has one range and takes a slice of it)
     const int slice_rows = p.split_tiles ? min(p.seg_rows[0] - tile0 * PBN, p.split_tiles * PBN) : 0;
     auto seg_rows = [&](int s) { return p.split_tiles ? slice_rows : p.seg_rows[s]; };
     int n_tiles = 0;   // key tiles over all segments
     for (int s = 0; s < p.segments; s++) n_tiles += (seg_rows(s) + PBN - 1) / PBN;
+    // Steps of query tiles A and B. The last CTA of a sequence may have no tile B; a causal tile ends
+    // at its own diagonal. n_tiles: steps of the CTA.
+    const bool has_b = q_row0 + PBM < p.lq;
+    const int steps_a = CAUSAL ? min(n_tiles, q_row0 / PBN + 1) : n_tiles;
+    const int steps_b = !has_b ? 0 : CAUSAL ? min(n_tiles, q_row0 / PBN + 2) : n_tiles;
+    if (CAUSAL) n_tiles = max(steps_a, steps_b);
 
     if (tid == 0) {
         mbar_init(bar_q_full, 1);
@@ -150,21 +174,20 @@ attn_tc5_pair_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
     if (skip_launch) {
         // straight to the teardown
     } else if (warp >= 8) {
-    warpgroup_reg_dec<88>();
+    warpgroup_reg_dec<PAIR_OTHER_REGS>();
     if (warp == 8) {
         // ------------------------------ TMA producer ------------------------------
         if (lane == 0) {
             tma_prefetch_desc(&map_q);
-            mbar_arrive_expect_tx(bar_q_full, PAIR_Q_BYTES);
-            for (int t = 0; t < 2; t++) {
-                const uint32_t dst = q_smem + t * (PAIR_Q_BYTES / 2);
-                tma_load_4d(dst, &map_q, bar_q_full, 0, head, q_row0 + t * PBM, batch);
-                tma_load_4d(dst + PAIR_HALF_BYTES, &map_q, bar_q_full, 64, head, q_row0 + t * PBM, batch);
-            }
+            mbar_arrive_expect_tx(bar_q_full, (has_b ? 2 : 1) * Cfg::Q_TILE_BYTES);
+            for (int t = 0; t < (has_b ? 2 : 1); t++)
+                for (int h = 0; h < Cfg::HALVES; h++)
+                    tma_load_4d(q_smem + t * Cfg::Q_TILE_BYTES + h * PAIR_HALF_BYTES, &map_q, bar_q_full, 64 * h, head,
+                                q_row0 + t * PBM, batch);
             int idx = 0;   // tile number: even = K, odd = V
             bool ok = true;
             for (int seg = 0; ok && seg < p.segments; seg++) {
-                const int tiles = (seg_rows(seg) + PBN - 1) / PBN;
+                const int tiles = CAUSAL ? n_tiles : (seg_rows(seg) + PBN - 1) / PBN;
                 for (int tile = 0; ok && tile < tiles; tile++) {
                     for (int which = 0; which < 2; which++, idx++) {
                         const int s = idx % ST, use = idx / ST;
@@ -172,11 +195,12 @@ attn_tc5_pair_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
                             ok = false;
                             break;
                         }
-                        const uint32_t dst = ring + s * PAIR_TILE_BYTES;
+                        const uint32_t dst = ring + s * Cfg::TILE_BYTES;
                         const void *map = which ? (const void *)&kv.v[seg] : (const void *)&kv.k[seg];
-                        mbar_arrive_expect_tx(bar_full(s), PAIR_TILE_BYTES);
-                        tma_load_4d(dst, map, bar_full(s), 0, kv_head, (tile0 + tile) * PBN, batch);
-                        tma_load_4d(dst + PAIR_HALF_BYTES, map, bar_full(s), 64, kv_head, (tile0 + tile) * PBN, batch);
+                        mbar_arrive_expect_tx(bar_full(s), Cfg::TILE_BYTES);
+                        for (int h = 0; h < Cfg::HALVES; h++)
+                            tma_load_4d(dst + h * PAIR_HALF_BYTES, map, bar_full(s), 64 * h, kv_head,
+                                        (tile0 + tile) * PBN, batch);
                     }
                 }
             }
@@ -188,14 +212,14 @@ attn_tc5_pair_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
         // uniform register in front of each MMA.
         {
             const bool leader = elect_one();
-            constexpr uint32_t idesc_qk = mma_idesc(PBM, PBN, 1, 0);
-            constexpr uint32_t idesc_pv = mma_idesc(PBM, PHD, 1, 1);
+            constexpr uint32_t idesc_qk = mma_idesc(PBM, PBN, F16 ? 0 : 1, 0);
+            constexpr uint32_t idesc_pv = mma_idesc(PBM, HD, F16 ? 0 : 1, 1);
             // Descriptors are built once (Q) or once per stage (K, V); a K-step only adds to
             // the low word: +2 per 32 bytes inside a 64-column half, +1024 for the second half
             // (16 KB), +128 per 16 V rows (2 KB).
             uint32_t q_lo[2], q_hi[2];
             for (int t = 0; t < 2; t++) {
-                const uint64_t d = smem_desc_sw128(q_smem + t * (PAIR_Q_BYTES / 2), 16, 1024);
+                const uint64_t d = smem_desc_sw128(q_smem + t * Cfg::Q_TILE_BYTES, 16, 1024);
                 q_lo[t] = (uint32_t)d;
                 q_hi[t] = (uint32_t)(d >> 32);
             }
@@ -204,10 +228,10 @@ attn_tc5_pair_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
             const uint32_t k_hi = (uint32_t)(k_proto >> 32), v_hi = (uint32_t)(v_proto >> 32);
             const uint32_t k_ring_lo = (uint32_t)k_proto, v_ring_lo = (uint32_t)v_proto;  // LBO lives in the low word
             auto issue_qk = [&](int j, int t) {   // S_t = Q_t . K_j^T
-                const uint32_t k_lo = k_ring_lo + ((2 * j) % ST) * (PAIR_TILE_BYTES >> 4);
+                const uint32_t k_lo = k_ring_lo + ((2 * j) % ST) * (Cfg::TILE_BYTES >> 4);
                 if (leader) {
 #pragma unroll
-                    for (int kk = 0; kk < PHD / 16; kk++) {
+                    for (int kk = 0; kk < HD / 16; kk++) {
                         const uint32_t off = (kk / 4) * (PAIR_HALF_BYTES >> 4) + (kk % 4) * 2;
                         mma_ss_words(tmem + t * PBN, q_lo[t] + off, q_hi[t], k_lo + off, k_hi, idesc_qk,
                                      kk > 0);
@@ -217,13 +241,13 @@ attn_tc5_pair_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
                 __syncwarp();
             };
             auto issue_pv = [&](int j, int t, int piece) {   // O_t += P_t . V_j over keys 0-63, 64-95 or 96-127
-                const uint32_t v_lo = v_ring_lo + ((2 * j + 1) % ST) * (PAIR_TILE_BYTES >> 4);
+                const uint32_t v_lo = v_ring_lo + ((2 * j + 1) % ST) * (Cfg::TILE_BYTES >> 4);
                 const int first = piece == 0 ? 0 : piece == 1 ? 4 : 6, last = piece == 0 ? 4 : piece == 1 ? 6 : 8;
                 if (leader) {
 #pragma unroll
                     for (int kk = 0; kk < 8; kk++)
                         if (kk >= first && kk < last)
-                            mma_ts_words(tmem + PAIR_O_COL + t * PHD, tmem + t * PBN + kk * 8,
+                            mma_ts_words(tmem + PAIR_O_COL + t * HD, tmem + t * PBN + kk * 8,
                                          v_lo + kk * (2048 >> 4), v_hi, idesc_pv, (j > 0) || (kk > 0));
                 }
                 __syncwarp();
@@ -240,41 +264,48 @@ attn_tc5_pair_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
             if (alive) {
                 tc5_fence_after();
                 issue_qk(0, 0);
-                issue_qk(0, 1);
+                if (steps_b > 0) issue_qk(0, 1);
                 release(0);
             }
             for (int j = 0; alive && j < n_tiles; j++) {
                 const bool more = j + 1 < n_tiles;
-                {
-                    // P of tile A, and (through the ring watcher) V of this step and K of the next
-                    TRACE_T0();
-                    if (!mbar_wait_converged(bar_p_full(0, 0), j & 1, &abort_word)) break;
-                    TRACE_ADD(0);
-                }
-                tc5_fence_after();
-                {
-                    TRACE_T0();
-                    issue_pv(j, 0, 0);
-                    if (!mbar_wait_converged(bar_p_full(0, 1), j & 1, &abort_word)) break;
+                if (!CAUSAL || j < steps_a) {
+                    {
+                        // P of tile A, and (through the ring watcher) V of this step and K of the next
+                        TRACE_T0();
+                        if (!mbar_wait_converged(bar_p_full(0, 0), j & 1, &abort_word)) break;
+                        TRACE_ADD(0);
+                    }
                     tc5_fence_after();
-                    issue_pv(j, 0, 1);
-                    if (!mbar_wait_converged(bar_p_full(0, 2), j & 1, &abort_word)) break;
+                    {
+                        TRACE_T0();
+                        issue_pv(j, 0, 0);
+                        if (!mbar_wait_converged(bar_p_full(0, 1), j & 1, &abort_word)) break;
+                        tc5_fence_after();
+                        issue_pv(j, 0, 1);
+                        if (!mbar_wait_converged(bar_p_full(0, 2), j & 1, &abort_word)) break;
+                        tc5_fence_after();
+                        issue_pv(j, 0, 2);
+                        TRACE_ADD(4);
+                    }
+                    if (j + 1 < steps_a) {
+                        TRACE_T0();
+                        issue_qk(j + 1, 0);
+                        TRACE_ADD(5);
+                    }
+                } else {
+                    // tile A has passed its diagonal (its watcher is done): V of this step directly
+                    const int v = 2 * j + 1;
+                    if (!mbar_wait_converged(bar_full(v % ST), (v / ST) & 1, &abort_word)) break;
                     tc5_fence_after();
-                    issue_pv(j, 0, 2);
-                    TRACE_ADD(4);
                 }
-                if (more) {
-                    TRACE_T0();
-                    issue_qk(j + 1, 0);
-                    TRACE_ADD(5);
-                }
-                {
-                    TRACE_T0();
-                    if (!mbar_wait_converged(bar_p_full(1, 0), j & 1, &abort_word)) break;
-                    TRACE_ADD(3);
-                }
-                tc5_fence_after();
-                {
+                if (j < steps_b) {
+                    {
+                        TRACE_T0();
+                        if (!mbar_wait_converged(bar_p_full(1, 0), j & 1, &abort_word)) break;
+                        TRACE_ADD(3);
+                    }
+                    tc5_fence_after();
                     TRACE_T0();
                     issue_pv(j, 1, 0);
                     if (!mbar_wait_converged(bar_p_full(1, 1), j & 1, &abort_word)) break;
@@ -283,12 +314,12 @@ attn_tc5_pair_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
                     if (!mbar_wait_converged(bar_p_full(1, 2), j & 1, &abort_word)) break;
                     tc5_fence_after();
                     issue_pv(j, 1, 2);
-                    release(2 * j + 1);
                     TRACE_ADD(6);
                 }
+                release(2 * j + 1);
                 if (more) {
                     TRACE_T0();
-                    issue_qk(j + 1, 1);
+                    if (j + 1 < steps_b) issue_qk(j + 1, 1);
                     release(2 * j + 2);
                     TRACE_ADD(7);
                 } else if (leader) {
@@ -316,7 +347,7 @@ attn_tc5_pair_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
         if (lane == 0) {
             // One arrival per phase of P_A's barrier: the next tiles are often there before the
             // softmax threads are done, so wait for the phase to end before arriving again.
-            for (int g = 0; g < n_tiles; g++) {
+            for (int g = 0; g < steps_a; g++) {
                 const int v = 2 * g + 1, k = 2 * g + 2;
                 if (!mbar_wait_parked(bar_full(v % ST), (v / ST) & 1, &abort_word)) break;
                 if (g + 1 < n_tiles && !mbar_wait_parked(bar_full(k % ST), (k / ST) & 1, &abort_word)) break;
@@ -326,26 +357,93 @@ attn_tc5_pair_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
         }
     }
     } else {
-        warpgroup_reg_inc<208>();
+        warpgroup_reg_inc<PAIR_SOFTMAX_REGS>();
         // ------------------------------ online softmax ------------------------------
         const int t = warp >> 2;                // which query tile
         const int r = tid & 127;                // row inside the tile == TMEM lane
         const uint32_t lane_base = (uint32_t)((warp & 3) * 32) << 16;
         const uint32_t s_addr = tmem + lane_base + t * PBN;
-        const uint32_t o_addr = tmem + lane_base + PAIR_O_COL + t * PHD;
+        const uint32_t o_addr = tmem + lane_base + PAIR_O_COL + t * HD;
+        const int steps = t ? steps_b : steps_a;
         float m_ref = -INFINITY, l = 0.0f;
         bool alive = true;
 #ifdef H3B_TRACE
         long long g_pair_trace_local[8] = {};
         const long long trace_begin = clock64();
 #endif
+        // One step of this thread's row: scores from TMEM (the whole row in registers, one read pass),
+        // P back over them in three pieces. MASKED: only the first nvalid scores count.
+        auto softmax_step = [&](auto masked, int j, int nvalid) {
+            constexpr bool MASKED = decltype(masked)::value;
+            constexpr int POLY = MASKED ? 0 : Cfg::POLY;   // a masked score is -inf: exactly zero weight
+            uint32_t s0[32], s1[32], s2[32], s3[32];
+            tmem_ld32(s_addr, s0);
+            tmem_ld32(s_addr + 32, s1);
+            tmem_ld32(s_addr + 64, s2);
+            tmem_ld32(s_addr + 96, s3);
+            tmem_wait_ld();
+            if (MASKED) {
+                mask_chunk(s0, nvalid);
+                mask_chunk(s1, nvalid - 32);
+                mask_chunk(s2, nvalid - 64);
+                mask_chunk(s3, nvalid - 96);
+            }
+            float mx[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
+            max_chunk4(s0, mx);
+            max_chunk4(s1, mx);
+            max_chunk4(s2, mx);
+            max_chunk4(s3, mx);
+            const float m_new = fmaxf(max3(m_ref, mx[0], mx[1]), fmaxf(mx[2], mx[3]));
+            const bool grow = (m_new - m_ref) * p.scale_log2 > PAIR_RESCALE_LOG2;
+            if (__any_sync(0xffffffffu, grow)) {
+                const float alpha = grow ? fast_exp2((m_ref - m_new) * p.scale_log2) : 1.0f;
+                if (grow) m_ref = m_new;
+                l *= alpha;
+                if (j > 0) {   // PV(j-1) is complete: S(j)'s commit covered it
+#pragma unroll
+                    for (int c = 0; c < HD / 32; c++) {
+                        uint32_t v[32];
+                        tmem_ld32(o_addr + c * 32, v);
+                        tmem_wait_ld();
+#pragma unroll
+                        for (int i = 0; i < 32; i++)
+                            v[i] = __float_as_uint(__uint_as_float(v[i]) * alpha);
+                        tmem_st32(o_addr + c * 32, v);
+                    }
+                    tmem_wait_st();
+                }
+            }
+            const float neg = -m_ref * p.scale_log2;
+            const float2 scale2 = make_float2(p.scale_log2, p.scale_log2);
+            const float2 neg2 = make_float2(neg, neg);
+            float2 sum0 = make_float2(0.f, 0.f), sum1 = make_float2(0.f, 0.f);
+            uint32_t packed[16];
+            exp_chunk_mixed<POLY, F16>(s0, packed, scale2, neg2, sum0, sum1);
+            tmem_st16(s_addr, packed);
+            exp_chunk_mixed<POLY, F16>(s1, packed, scale2, neg2, sum0, sum1);
+            tmem_st16(s_addr + 16, packed);
+            tmem_wait_st();
+            tc5_fence_before();
+            mbar_arrive(bar_p_full(t, 0));
+            exp_chunk_mixed<POLY, F16>(s2, packed, scale2, neg2, sum0, sum1);
+            tmem_st16(s_addr + 32, packed);
+            tmem_wait_st();
+            tc5_fence_before();
+            mbar_arrive(bar_p_full(t, 1));
+            exp_chunk_mixed<POLY, F16>(s3, packed, scale2, neg2, sum0, sum1);
+            tmem_st16(s_addr + 48, packed);
+            l += (sum0.x + sum0.y) + (sum1.x + sum1.y);
+            tmem_wait_st();
+            tc5_fence_before();
+            mbar_arrive(bar_p_full(t, 2));
+        };
         int seg = 0, seg_tile = 0;   // which segment, which tile of it, step j is
-        for (int j = 0; j < n_tiles; j++) {
+        for (int j = 0; j < steps; j++) {
             while (seg_tile * PBN >= seg_rows(seg)) {
                 seg++;
                 seg_tile = 0;
             }
-            const int nvalid = min(PBN, seg_rows(seg) - seg_tile * PBN);
+            const int in_range = min(PBN, seg_rows(seg) - seg_tile * PBN);
             seg_tile++;
             {
                 TRACE_T0();
@@ -357,92 +455,12 @@ attn_tc5_pair_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
 #ifdef H3B_TRACE
             const long long trace_work = clock64();
 #endif
-            bool first_half_out = false, second_piece_out = false;
-            if (nvalid >= PBN) {
-                // the whole row of scores in registers: one TMEM read pass
-                uint32_t s0[32], s1[32], s2[32], s3[32];
-                tmem_ld32(s_addr, s0);
-                tmem_ld32(s_addr + 32, s1);
-                tmem_ld32(s_addr + 64, s2);
-                tmem_ld32(s_addr + 96, s3);
-                tmem_wait_ld();
-                float mx[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
-                max_chunk4(s0, mx);
-                max_chunk4(s1, mx);
-                max_chunk4(s2, mx);
-                max_chunk4(s3, mx);
-                const float m_new = fmaxf(max3(m_ref, mx[0], mx[1]), fmaxf(mx[2], mx[3]));
-                const bool grow = (m_new - m_ref) * p.scale_log2 > PAIR_RESCALE_LOG2;
-                if (__any_sync(0xffffffffu, grow)) {
-                    const float alpha = grow ? fast_exp2((m_ref - m_new) * p.scale_log2) : 1.0f;
-                    if (grow) m_ref = m_new;
-                    l *= alpha;
-                    if (j > 0) {   // PV(j-1) is complete: S(j)'s commit covered it
-#pragma unroll
-                        for (int c = 0; c < PHD / 32; c++) {
-                            uint32_t v[32];
-                            tmem_ld32(o_addr + c * 32, v);
-                            tmem_wait_ld();
-#pragma unroll
-                            for (int i = 0; i < 32; i++)
-                                v[i] = __float_as_uint(__uint_as_float(v[i]) * alpha);
-                            tmem_st32(o_addr + c * 32, v);
-                        }
-                        tmem_wait_st();
-                    }
-                }
-                const float neg = -m_ref * p.scale_log2;
-                const float2 scale2 = make_float2(p.scale_log2, p.scale_log2);
-                const float2 neg2 = make_float2(neg, neg);
-                float2 sum0 = make_float2(0.f, 0.f), sum1 = make_float2(0.f, 0.f);
-                uint32_t packed[16];
-                exp_chunk_mixed<PAIR_POLY_EVERY>(s0, packed, scale2, neg2, sum0, sum1);
-                tmem_st16(s_addr, packed);
-                exp_chunk_mixed<PAIR_POLY_EVERY>(s1, packed, scale2, neg2, sum0, sum1);
-                tmem_st16(s_addr + 16, packed);
-                tmem_wait_st();
-                tc5_fence_before();
-                mbar_arrive(bar_p_full(t, 0));
-                first_half_out = true;
-                exp_chunk_mixed<PAIR_POLY_EVERY>(s2, packed, scale2, neg2, sum0, sum1);
-                tmem_st16(s_addr + 32, packed);
-                tmem_wait_st();
-                tc5_fence_before();
-                mbar_arrive(bar_p_full(t, 1));
-                second_piece_out = true;
-                exp_chunk_mixed<PAIR_POLY_EVERY>(s3, packed, scale2, neg2, sum0, sum1);
-                tmem_st16(s_addr + 48, packed);
-                l += (sum0.x + sum0.y) + (sum1.x + sum1.y);
-            } else {
-                // ragged last tile: masked two-pass path
-                const float mx = row_max_masked<PBN>(s_addr, nvalid);
-                const float m_new = fmaxf(m_ref, mx);
-                const bool grow = (m_new - m_ref) * p.scale_log2 > PAIR_RESCALE_LOG2;
-                if (__any_sync(0xffffffffu, grow)) {
-                    const float alpha = grow ? fast_exp2((m_ref - m_new) * p.scale_log2) : 1.0f;
-                    if (grow) m_ref = m_new;
-                    l *= alpha;
-                    if (j > 0) {   // PV(j-1) is complete: S(j)'s commit covered it
-#pragma unroll
-                        for (int c = 0; c < PHD / 32; c++) {
-                            uint32_t v[32];
-                            tmem_ld32(o_addr + c * 32, v);
-                            tmem_wait_ld();
-#pragma unroll
-                            for (int i = 0; i < 32; i++)
-                                v[i] = __float_as_uint(__uint_as_float(v[i]) * alpha);
-                            tmem_st32(o_addr + c * 32, v);
-                        }
-                        tmem_wait_st();
-                    }
-                }
-                l += exp_store_masked<PBN>(s_addr, s_addr, p.scale_log2, -m_ref * p.scale_log2, nvalid);
-            }
-            tmem_wait_st();
-            tc5_fence_before();
-            if (!first_half_out) mbar_arrive(bar_p_full(t, 0));
-            if (!second_piece_out) mbar_arrive(bar_p_full(t, 1));
-            mbar_arrive(bar_p_full(t, 2));
+            // keys up to this row's own, counted from the tile's first key; least[warp] = its lane 0
+            const int causal_first = q_row0 + t * PBM + (warp & 3) * 32 + 1 - j * PBN;
+            if (min(in_range, CAUSAL ? causal_first : PBN) >= PBN)
+                softmax_step(std::false_type{}, j, PBN);
+            else
+                softmax_step(std::true_type{}, j, CAUSAL ? min(in_range, causal_first + lane) : in_range);
 #ifdef H3B_TRACE
             g_pair_trace_local[1] += clock64() - trace_work;
 #endif
@@ -456,25 +474,26 @@ attn_tc5_pair_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
 #endif
 
         // -------- epilogue: O / l -> bf16, straight to global memory --------
+        alive = alive && steps > 0;
         if (alive) alive = __all_sync(0xffffffffu, mbar_wait(bar_pv_done, 0, &abort_word));
         if (alive) {
             tc5_fence_after();
             const float inv = 1.0f / l;
             const int row = q_row0 + t * PBM + r;
             const bool store = row < p.lq;
-            __nv_bfloat16 *dst;
+            uint16_t *dst;
             if (p.rows_per_rank) {
                 // this row belongs to another rank's row shard: store it there, in place
                 const unsigned owner = (unsigned)row / p.rows_per_rank, local = (unsigned)row % p.rows_per_rank;
                 dst = p.peer_out[store ? owner : 0] +
-                      ((size_t)local * p.total_heads + (size_t)p.rank * p.heads + head) * PHD;
+                      ((size_t)local * p.total_heads + (size_t)p.rank * p.heads + head) * HD;
             } else {
-                dst = p.out + (((size_t)out_batch * p.lq + row) * p.heads + head) * PHD;
+                dst = p.out + (((size_t)out_batch * p.lq + row) * p.heads + head) * HD;
             }
             if (store && p.lse)
                 p.lse[((size_t)out_batch * p.heads + head) * p.lq + row] = m_ref * p.scale + __logf(l);
 #pragma unroll
-            for (int c = 0; c < PHD / 32; c++) {
+            for (int c = 0; c < HD / 32; c++) {
                 uint32_t v[32];
                 tmem_ld32(o_addr + c * 32, v);
                 tmem_wait_ld();
@@ -483,10 +502,10 @@ attn_tc5_pair_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
 #pragma unroll
                     for (int i = 0; i < 4; i++) {
                         uint4 w;
-                        w.x = pack_bf16(__uint_as_float(v[i * 8 + 0]) * inv, __uint_as_float(v[i * 8 + 1]) * inv);
-                        w.y = pack_bf16(__uint_as_float(v[i * 8 + 2]) * inv, __uint_as_float(v[i * 8 + 3]) * inv);
-                        w.z = pack_bf16(__uint_as_float(v[i * 8 + 4]) * inv, __uint_as_float(v[i * 8 + 5]) * inv);
-                        w.w = pack_bf16(__uint_as_float(v[i * 8 + 6]) * inv, __uint_as_float(v[i * 8 + 7]) * inv);
+                        w.x = pack_p<F16>(__uint_as_float(v[i * 8 + 0]) * inv, __uint_as_float(v[i * 8 + 1]) * inv);
+                        w.y = pack_p<F16>(__uint_as_float(v[i * 8 + 2]) * inv, __uint_as_float(v[i * 8 + 3]) * inv);
+                        w.z = pack_p<F16>(__uint_as_float(v[i * 8 + 4]) * inv, __uint_as_float(v[i * 8 + 5]) * inv);
+                        w.w = pack_p<F16>(__uint_as_float(v[i * 8 + 6]) * inv, __uint_as_float(v[i * 8 + 7]) * inv);
                         d4[i] = w;
                     }
                 }
@@ -552,23 +571,46 @@ cudaError_t attn_merge_splits(void *out, float *lse_out, const void *partial, co
     return cudaGetLastError();
 }
 
-cudaError_t attn_dense_tc5_pair(const CUtensorMap_st *mq, const CUtensorMap_st *mk,
-                                const CUtensorMap_st *mv, void *out, float *lse, unsigned batch,
-                                unsigned lq, unsigned lk, unsigned heads, unsigned kv_heads,
-                                float scale, int *status, cudaStream_t stream, const PeerOutput *peer,
-                                unsigned segments, const unsigned *segment_rows, unsigned split_tiles) {
+namespace {
+
+template <int HD, bool F16, bool CAUSAL>
+cudaError_t launch_pair(const CUtensorMap &mq, const PairKvMaps &kv, const PairParams &p, unsigned slices,
+                        cudaStream_t stream) {
+    auto kernel = attn_tc5_pair_kernel<HD, F16, CAUSAL>;
     static thread_local int configured_device = -1;
     int device = 0;
     cudaError_t e = cudaGetDevice(&device);
     if (e != cudaSuccess) return e;
     if (configured_device != device) {
-        e = cudaFuncSetAttribute(attn_tc5_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 PAIR_SMEM_BYTES);
+        // setmaxnreg moves registers inside what the CTA was given at launch; a build that was given
+        // fewer would wait for them for ever, so it is refused here
+        cudaFuncAttributes attributes{};
+        if ((e = cudaFuncGetAttributes(&attributes, kernel)) != cudaSuccess) return e;
+        if (attributes.numRegs * PAIR_THREADS < PAIR_SOFTMAX_REGS * 256 + PAIR_OTHER_REGS * 128)
+            return cudaErrorInvalidConfiguration;
+        e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, PairConfig<HD>::SMEM_BYTES);
         if (e != cudaSuccess) return e;
         configured_device = device;
     }
+    const unsigned pairs = ((unsigned)p.lq + 2 * PBM - 1) / (2 * PBM), heads = (unsigned)p.heads;
+    if (CAUSAL && pairs > 65535u) return cudaErrorInvalidValue;
+    const dim3 grid = CAUSAL ? dim3(heads, pairs, slices) : dim3(pairs, heads, slices);
+    kernel<<<grid, PAIR_THREADS, PairConfig<HD>::SMEM_BYTES, stream>>>(mq, kv, p);
+    return cudaGetLastError();
+}
+
+}  // namespace
+
+cudaError_t attn_dense_tc5_pair(const CUtensorMap_st *mq, const CUtensorMap_st *mk,
+                                const CUtensorMap_st *mv, void *out, float *lse, unsigned batch,
+                                unsigned lq, unsigned lk, unsigned heads, unsigned kv_heads,
+                                float scale, int *status, cudaStream_t stream, const PeerOutput *peer,
+                                unsigned segments, const unsigned *segment_rows, unsigned split_tiles,
+                                PairKind kind) {
     // mk / mv point to `segments` maps each; without a segment list: one range of lk rows
     if (segments > (unsigned)PAIR_MAX_SEGMENTS || (segments > 1 && batch != 1)) return cudaErrorInvalidValue;
+    if (kind != PairKind::BF16_D128 && (segments || split_tiles || peer)) return cudaErrorInvalidValue;
+    if (kind == PairKind::BF16_D128_CAUSAL && lq != lk) return cudaErrorInvalidValue;
     // split-KV: one key range, batch 1, no peer output; the slices ride on grid.z
     unsigned splits = 1;
     if (split_tiles) {
@@ -590,20 +632,23 @@ cudaError_t attn_dense_tc5_pair(const CUtensorMap_st *mq, const CUtensorMap_st *
     p.kv_heads = (int)kv_heads;
     p.scale = scale;
     p.scale_log2 = scale * 1.4426950408889634f;
-    p.out = static_cast<__nv_bfloat16 *>(out);
+    p.out = static_cast<uint16_t *>(out);
     p.lse = lse;
     p.status = status;
     p.split_tiles = (int)split_tiles;
     if (peer) {
         if (batch != 1 || !peer->rows_per_rank) return cudaErrorInvalidValue;
-        for (int i = 0; i < 16; i++) p.peer_out[i] = static_cast<__nv_bfloat16 *>(peer->base[i]);
+        for (int i = 0; i < 16; i++) p.peer_out[i] = static_cast<uint16_t *>(peer->base[i]);
         p.rows_per_rank = peer->rows_per_rank;
         p.rank = peer->rank;
         p.total_heads = peer->total_heads;
     }
-    dim3 grid((lq + 2 * PBM - 1) / (2 * PBM), heads, split_tiles ? splits : batch);
-    attn_tc5_pair_kernel<<<grid, PAIR_THREADS, PAIR_SMEM_BYTES, stream>>>(*mq, kv, p);
-    return cudaGetLastError();
+    const unsigned slices = split_tiles ? splits : batch;
+    switch (kind) {
+        case PairKind::BF16_D128_CAUSAL: return launch_pair<128, false, true>(*mq, kv, p, slices, stream);
+        case PairKind::F16_D64: return launch_pair<64, true, false>(*mq, kv, p, slices, stream);
+        default: return launch_pair<128, false, false>(*mq, kv, p, slices, stream);
+    }
 }
 
 }  // namespace h3b

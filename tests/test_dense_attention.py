@@ -160,6 +160,42 @@ def test_sdpa_f16_d64(gpu, oracle, L, H):
     assert_attention_close(got, want, max_abs=5e-3, rel_l2=0.004)
 
 
+@pytest.mark.parametrize("L", [1, 127, 128, 129, 255, 256, 257, 384, 385, 640, 1100])
+@pytest.mark.parametrize("shift", [0, 4])
+def test_causal_and_f16_at_tile_edges(gpu, oracle, L, shift):
+    """The causal and the fp16 head-dim-64 kernels where their tiles end (128-row tiles, two per CTA,
+    the diagonal inside or between them), and, with query and output 4 bytes off the 16-byte boundary,
+    the kernel that takes such tensors. fp16 limit: half an ulp of values up to 4 plus the rounding of
+    the weights (2^-12 each, averaged over the row)."""
+    from h3_omni_b200 import native
+    data, stream = gpu.lib.h3b_tensor_data, gpu.lib.h3b_gpu_stream(gpu.gpu)
+    pad = shift // 2
+
+    def shifted(x, dtype=None):
+        return data(gpu.tensor(np.concatenate([np.zeros(pad, np.uint16), x.ravel()]), dtype)) + shift
+
+    B, H, KH = 2, 6, 2
+    q = oracle.normal_bf16((B, L, H, 128), 10 + L)
+    k, v = (oracle.normal_bf16((B, L, KH, 128), 20 + L + i) for i in range(2))
+    ty = gpu.tensor(np.full(q.size + pad, 0x7fc0, dtype=np.uint16))
+    tl = gpu.tensor(np.zeros((B, H, L), dtype=np.float32))
+    gpu.raw("h3_flash_bf16", data(ty) + shift, shifted(q), data(gpu.tensor(k)), data(gpu.tensor(v)), data(tl), B, L, H,
+            KH, SCALE, True, stream)
+    want, _, want_lse = oracle.attention(q, k, v, SCALE, causal=True, want_lse=True)
+    assert_attention_close(oracle.from_bf16(gpu.read(ty, q.size + pad)[pad:].reshape(q.shape)), want)
+    assert np.abs(gpu.read(tl, (B, H, L), np.float32) - want_lse).max() < 2e-3
+
+    rng = np.random.default_rng(L)
+    q, k, v = (oracle.to_f16(rng.standard_normal((B, L, 3, 64))) for _ in range(3))
+    ty = gpu.tensor(np.full(q.size + pad, 0x7e00, dtype=np.uint16), native.F16)
+    gpu.raw("h3_flash3_f16_d64", data(ty) + shift, shifted(q, native.F16), data(gpu.tensor(k, native.F16)),
+            data(gpu.tensor(v, native.F16)), None, B, L, 3, 0.125, stream)
+    want, _ = oracle.attention(q, k, v, 0.125, elem="f16")
+    assert_attention_close(oracle.from_f16(gpu.read(ty, q.size + pad)[pad:].reshape(q.shape)), want, max_abs=2e-3,
+                           rel_l2=0.001)
+    assert gpu.device_status() == 0
+
+
 def test_sdpa_rejects_bad_arguments(gpu, oracle):
     """Error behaviour of the primitive layer: 0 + message, no launch."""
     q = gpu.tensor(oracle.normal_bf16((4, 2, 128), 1))
