@@ -267,9 +267,13 @@ attn_tc5_pair_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
                 if (steps_b > 0) issue_qk(0, 1);
                 release(0);
             }
+            // EVEN: both tiles take every step (the hot case, straight-line: a branch in this warp's loop
+            // leaves the tensor pipe idle, 1.7 % of a long call). Otherwise each tile has its own number.
+            auto walk = [&](auto even) {
+            constexpr bool EVEN = decltype(even)::value;
             for (int j = 0; alive && j < n_tiles; j++) {
                 const bool more = j + 1 < n_tiles;
-                if (!CAUSAL || j < steps_a) {
+                if (EVEN || j < steps_a) {
                     {
                         // P of tile A, and (through the ring watcher) V of this step and K of the next
                         TRACE_T0();
@@ -288,7 +292,7 @@ attn_tc5_pair_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
                         issue_pv(j, 0, 2);
                         TRACE_ADD(4);
                     }
-                    if (j + 1 < steps_a) {
+                    if (EVEN ? more : j + 1 < steps_a) {
                         TRACE_T0();
                         issue_qk(j + 1, 0);
                         TRACE_ADD(5);
@@ -299,7 +303,7 @@ attn_tc5_pair_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
                     if (!mbar_wait_converged(bar_full(v % ST), (v / ST) & 1, &abort_word)) break;
                     tc5_fence_after();
                 }
-                if (j < steps_b) {
+                if (EVEN || j < steps_b) {
                     {
                         TRACE_T0();
                         if (!mbar_wait_converged(bar_p_full(1, 0), j & 1, &abort_word)) break;
@@ -319,7 +323,7 @@ attn_tc5_pair_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
                 release(2 * j + 1);
                 if (more) {
                     TRACE_T0();
-                    if (j + 1 < steps_b) issue_qk(j + 1, 1);
+                    if (EVEN || j + 1 < steps_b) issue_qk(j + 1, 1);
                     release(2 * j + 2);
                     TRACE_ADD(7);
                 } else if (leader) {
@@ -327,6 +331,9 @@ attn_tc5_pair_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
                 }
                 __syncwarp();
             }
+            };
+            if (!CAUSAL && has_b) walk(std::true_type{});
+            else walk(std::false_type{});
 #ifdef H3B_TRACE
             if (blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0 && lane == 0) {
                 g_pair_trace[0] = clock64() - trace_begin;   // MMA thread: whole walk
@@ -389,12 +396,13 @@ attn_tc5_pair_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
                 mask_chunk(s3, nvalid - 96);
             }
             float mx[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
-            max_chunk4(s0, mx);
-            max_chunk4(s1, mx);
-            max_chunk4(s2, mx);
-            max_chunk4(s3, mx);
-            const float m_new = fmaxf(max3(m_ref, mx[0], mx[1]), fmaxf(mx[2], mx[3]));
-            const bool grow = (m_new - m_ref) * p.scale_log2 > PAIR_RESCALE_LOG2;
+            max_chunk4<true>(s0, mx);
+            max_chunk4<true>(s1, mx);
+            max_chunk4<true>(s2, mx);
+            max_chunk4<true>(s3, mx);
+            // A NaN score makes the maximum NaN, and that the row: not every column's exponential keeps it.
+            const float m_new = max3<true>(max3<true>(m_ref, mx[0], mx[1]), mx[2], mx[3]);
+            const bool grow = !((m_new - m_ref) * p.scale_log2 <= PAIR_RESCALE_LOG2);
             if (__any_sync(0xffffffffu, grow)) {
                 const float alpha = grow ? fast_exp2((m_ref - m_new) * p.scale_log2) : 1.0f;
                 if (grow) m_ref = m_new;

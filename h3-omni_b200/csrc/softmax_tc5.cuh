@@ -6,9 +6,12 @@
 
 namespace h3b {
 
+// The largest of three; with NAN_COUNTS a NaN if any of them is one, otherwise NaNs lose.
+template <bool NAN_COUNTS = false>
 __device__ __forceinline__ float max3(float a, float b, float c) {
     float d;
-    asm("max.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
+    if constexpr (NAN_COUNTS) asm("max.NaN.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
+    else asm("max.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
     return d;
 }
 __device__ __forceinline__ void max_chunk(const uint32_t (&v)[32], float &m0, float &m1) {
@@ -20,12 +23,13 @@ __device__ __forceinline__ void max_chunk(const uint32_t (&v)[32], float &m0, fl
 }
 // The same over four independent chains (a lone warp on its scheduler is bound by the latency of
 // the chain, not by issue slots).
+template <bool NAN_COUNTS = false>
 __device__ __forceinline__ void max_chunk4(const uint32_t (&v)[32], float (&m)[4]) {
 #pragma unroll
     for (int i = 0; i < 32; i += 8) {
 #pragma unroll
         for (int k = 0; k < 4; k++)
-            m[k] = max3(m[k], __uint_as_float(v[i + 2 * k]), __uint_as_float(v[i + 2 * k + 1]));
+            m[k] = max3<NAN_COUNTS>(m[k], __uint_as_float(v[i + 2 * k]), __uint_as_float(v[i + 2 * k + 1]));
     }
 }
 // Scores from number nvalid on become -inf.

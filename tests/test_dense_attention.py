@@ -196,6 +196,28 @@ def test_causal_and_f16_at_tile_edges(gpu, oracle, L, shift):
     assert gpu.device_status() == 0
 
 
+@pytest.mark.parametrize("column", [0, 2, 66])
+def test_not_a_number_in_a_key_reaches_its_rows(gpu, oracle, column):
+    """A NaN key makes every row that attends it NaN, whichever unit takes the exponential of its column."""
+    from h3_omni_b200 import native
+    data, stream = gpu.lib.h3b_tensor_data, gpu.lib.h3b_gpu_stream(gpu.gpu)
+    L, key = 400, 128 + column
+    q, k, v = (oracle.normal_bf16((1, L, 2, 128), 30 + i) for i in range(3))
+    k[0, key, :, 3] = 0x7fc0
+    for causal in (False, True):
+        ty = gpu.tensor(np.zeros(q.shape, dtype=np.uint16))
+        gpu.raw("h3_flash_bf16", *[data(t) for t in (ty, gpu.tensor(q), gpu.tensor(k), gpu.tensor(v))], None, 1, L, 2, 2,
+                SCALE, causal, stream)
+        out = oracle.from_bf16(gpu.read(ty, q.shape))[0]
+        first = key if causal else 0
+        assert np.isnan(out[first:]).all() and np.isfinite(out[:first]).all()
+    q, k, v = (oracle.to_f16(np.random.default_rng(40 + i).standard_normal((1, L, 2, 64))) for i in range(3))
+    k[0, key, :, 3] = 0x7e00
+    ty = gpu.tensor(np.zeros(q.shape, dtype=np.uint16), native.F16)
+    gpu.raw("h3_flash3_f16_d64", data(ty), *[data(gpu.tensor(x, native.F16)) for x in (q, k, v)], None, 1, L, 2, 0.125, stream)
+    assert np.isnan(oracle.from_f16(gpu.read(ty, q.shape))).all()
+
+
 def test_sdpa_rejects_bad_arguments(gpu, oracle):
     """Error behaviour of the primitive layer: 0 + message, no launch."""
     q = gpu.tensor(oracle.normal_bf16((4, 2, 128), 1))
