@@ -45,7 +45,6 @@ constexpr int PAIR_THREADS = 384;                  // three warpgroups: softmax 
 constexpr int PAIR_SOFTMAX_REGS = 208, PAIR_OTHER_REGS = 88;   // what setmaxnreg leaves the warpgroups with
 constexpr int PAIR_HALF_BYTES = PBN * 128;          // one 64-column half of a tile
 constexpr int PAIR_O_COL = 256;
-constexpr float PAIR_RESCALE_LOG2 = 8.0f;
 
 // What depends on the head dimension. HD = 128: 64 KB of Q and five slots of 32 KB. HD = 64: half
 // of each, so the ring gets eight slots; the products take half the time, the softmax the same, so
@@ -104,6 +103,11 @@ attn_tc5_pair_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
                      const PairParams p) {
     using Cfg = PairConfig<HD>;
     constexpr int ST = Cfg::STAGES;
+    // How far a row's maximum may run ahead of its reference before O is rescaled. The long bf16 walks of the
+    // non-causal kernel leave it at 2^8. The causal and the fp16 kernel follow the maximum: a row's largest
+    // weight is then exactly 1, and their error against 64 bits that of the mma.sync kernel they replace (2 to 4 %
+    // more with 2^8: a short row has few weights, and fp16 ones are otherwise as exact as the result).
+    constexpr float RESCALE_LOG2 = CAUSAL || F16 ? 0.0f : 8.0f;
     extern __shared__ uint8_t smem_raw[];
     __shared__ uint64_t bars[1 + 2 * ST + 9];
     __shared__ uint32_t tmem_slot;
@@ -402,7 +406,7 @@ attn_tc5_pair_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
             max_chunk4<true>(s3, mx);
             // A NaN score makes the maximum NaN, and that the row: not every column's exponential keeps it.
             const float m_new = max3<true>(max3<true>(m_ref, mx[0], mx[1]), mx[2], mx[3]);
-            const bool grow = !((m_new - m_ref) * p.scale_log2 <= PAIR_RESCALE_LOG2);
+            const bool grow = !((m_new - m_ref) * p.scale_log2 <= RESCALE_LOG2);
             if (__any_sync(0xffffffffu, grow)) {
                 const float alpha = grow ? fast_exp2((m_ref - m_new) * p.scale_log2) : 1.0f;
                 if (grow) m_ref = m_new;
