@@ -7,9 +7,14 @@
 //   gated  = bf16(residual + bf16(y * gate[map[row]][gate_slot]))         (h3_gate_bf16)
 //   output = bf16(bf16(bf16(gated * rsqrt(mean(gated^2) + eps) * norm_w) * bf16(1 + scale)) + shift)   (h3_adaln_bf16)
 //
-// Kernel 1 is a persistent tcgen05 GEMM (TMA-fed, 128 x 256 output tiles, two accumulators in
-// TMEM so the epilogue of one tile runs under the MMAs of the next) whose epilogue applies gate and
-// residual to the fp32 accumulators and writes `gated`; y is never written to memory. Kernel 2 is
+// Kernel 1 is a persistent tcgen05 GEMM whose epilogue applies gate and residual to the fp32 accumulators
+// and writes `gated`; y is never written to memory. Two CTAs of a cluster, on two SMs, share an output
+// tile of 256 x GN (tcgen05 cta_group::2): each holds 128 rows of A and half of the rows of B, the even
+// one issues the MMAs of both. A k-step of 64 then takes 32 KB into each SM instead of the 48 KB of a
+// 128 x 256 tile of its own, and those fills are what bounded the one-SM form (94 B/clk asked of a path
+// that gave 73). Two accumulators in TMEM, so the epilogue of one tile runs under the MMAs of the next.
+// 15,400 x 7168 x 5376 with both kernels, back to back: 1169 us with one SM per tile, 1068 us so.
+// Kernel 2 is
 // the row-wise AdaLN in the reference's own operation order (it needs the whole gated row for the
 // RMS, so it cannot live in a tile epilogue). The A operand may be the window slot the attention
 // kernel gathered its output into, so at N GPUs nothing is copied between attention and projection.
@@ -22,11 +27,15 @@
 namespace h3b {
 namespace {
 
-constexpr int GM = 128, GN = 256, GK = 64;          // CTA tile; GK = one 128-byte swizzle row
-constexpr int G_STAGES = 4;
-constexpr int G_A_BYTES = GM * GK * 2, G_B_BYTES = GN * GK * 2, G_STAGE = G_A_BYTES + G_B_BYTES;   // 16 + 32 KB
-constexpr int G_SMEM = G_STAGES * G_STAGE + 1024;
+constexpr int GM = 128, GK = 64;                     // rows of A per CTA; GK = one 128-byte swizzle row
+constexpr int G_A_BYTES = GM * GK * 2;
 constexpr int G_THREADS = 192;                       // warps 0-3 epilogue, 4 TMA, 5 MMA
+template <int GN>
+struct ProjConfig {
+    static constexpr int B_BYTES = GN / 2 * GK * 2, STAGE = G_A_BYTES + B_BYTES;
+    static constexpr int STAGES = GN == 256 ? 6 : 8;
+    static constexpr int SMEM = STAGES * STAGE + 1024;
+};
 
 struct OutProjParams {
     const __nv_bfloat16 *residual, *modulation;
@@ -41,68 +50,138 @@ __device__ __forceinline__ float bf16_lo(uint32_t w) { return __uint_as_float(w 
 __device__ __forceinline__ float bf16_hi(uint32_t w) { return __uint_as_float(w & 0xffff0000u); }
 __device__ __forceinline__ float round_bf16(float x) { return __bfloat162float(__float2bfloat16_rn(x)); }
 
-__device__ __forceinline__ void tma_load_2d(uint32_t dst, const void *map, uint32_t bar, int c0, int c1) {
+// ---- the two CTAs of a pair ----
+__device__ __forceinline__ uint32_t cluster_rank() {
+    uint32_t r;
+    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+    return r;
+}
+__device__ __forceinline__ void cluster_sync() {
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// The address of this CTA's shared variable in CTA `rank` of the cluster.
+__device__ __forceinline__ uint32_t map_to_rank(uint32_t addr, uint32_t rank) {
+    uint32_t r;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
+    return r;
+}
+__device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_addr) {
+    asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
+}
+__device__ __forceinline__ bool mbar_try_wait_cluster(uint32_t bar, uint32_t parity) {
+    uint32_t done;
     asm volatile(
-        "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
-        ::"r"(dst), "l"(map), "r"(bar), "r"(c0), "r"(c1)
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(done)
+        : "r"(bar), "r"(parity)
+        : "memory");
+    return done != 0;
+}
+// Bounded wait of a converged warp for arrivals that may come from the other CTA.
+__device__ __forceinline__ bool mbar_wait_cluster(uint32_t bar, uint32_t parity, volatile int *abort_word) {
+    unsigned long long start = 0;
+    for (uint32_t spin = 0;; ++spin) {
+        if (__all_sync(0xffffffffu, mbar_try_wait_cluster(bar, parity))) return true;
+        if ((spin & 255u) == 255u) {
+            const unsigned long long now = global_timer_ns();
+            if (!start) start = now;
+            if (now - start > WAIT_LIMIT_NS) *abort_word = 1;
+            if (__any_sync(0xffffffffu, *abort_word != 0)) return false;
+        }
+    }
+}
+// A load into this CTA's shared memory that reports to a barrier of either CTA of the pair.
+__device__ __forceinline__ void tma_load_2d_pair(uint32_t dst, const void *map, uint32_t cluster_bar, int c0, int c1) {
+    asm volatile(
+        "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes "
+        "[%0], [%1, {%3, %4}], [%2];"
+        ::"r"(dst), "l"(map), "r"(cluster_bar), "r"(c0), "r"(c1)
+        : "memory");
+}
+__device__ __forceinline__ void mma_ss_pair(uint32_t d_tmem, uint32_t a_lo, uint32_t a_hi, uint32_t b_lo, uint32_t b_hi,
+                                            uint32_t idesc, uint32_t accumulate) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t.reg .b64 da, db;\n\t"
+        "mov.b64 da, {%1, %2};\n\tmov.b64 db, {%3, %4};\n\t"
+        "setp.ne.b32 p, %6, 0;\n\t"
+        "tcgen05.mma.cta_group::2.kind::f16 [%0], da, db, %5, p;\n\t}"
+        ::"r"(d_tmem), "r"(a_lo), "r"(a_hi), "r"(b_lo), "r"(b_hi), "r"(idesc), "r"(accumulate)
+        : "memory");
+}
+// One arrival on this barrier in both CTAs once every MMA issued so far by this thread has completed.
+__device__ __forceinline__ void mma_commit_pair(uint32_t bar) {
+    asm volatile(
+        "tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(bar),
+        "h"((uint16_t)3)
         : "memory");
 }
 
-__global__ void __launch_bounds__(G_THREADS, 1)
+template <int GN>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(G_THREADS, 1)
 out_proj_gate_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
                      const OutProjParams p) {
+    using Cfg = ProjConfig<GN>;
+    constexpr int ST = Cfg::STAGES;
     extern __shared__ uint8_t smem_raw[];
-    __shared__ uint64_t bars[2 * G_STAGES + 4];
+    __shared__ uint64_t bars[2 * ST + 4];
     __shared__ uint32_t tmem_slot;
     __shared__ int abort_word;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const uint32_t rank = cluster_rank();
     const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
     const uint32_t bar0 = smem_u32(bars);
-    auto bar_full = [&](int s) { return bar0 + 8u * s; };
-    auto bar_empty = [&](int s) { return bar0 + 8u * (G_STAGES + s); };
-    auto bar_acc_full = [&](int a) { return bar0 + 8u * (2 * G_STAGES + a); };
-    auto bar_acc_empty = [&](int a) { return bar0 + 8u * (2 * G_STAGES + 2 + a); };
+    auto bar_full = [&](int s) { return bar0 + 8u * s; };                       // the even CTA's count for both
+    auto bar_empty = [&](int s) { return bar0 + 8u * (ST + s); };
+    auto bar_acc_full = [&](int a) { return bar0 + 8u * (2 * ST + a); };
+    auto bar_acc_empty = [&](int a) { return bar0 + 8u * (2 * ST + 2 + a); };   // likewise
     if (tid == 0) {
-        for (int s = 0; s < G_STAGES; s++) {
+        for (int s = 0; s < ST; s++) {
             mbar_init(bar_full(s), 1);
             mbar_init(bar_empty(s), 1);
         }
         for (int a = 0; a < 2; a++) {
             mbar_init(bar_acc_full(a), 1);
-            mbar_init(bar_acc_empty(a), 128);
+            mbar_init(bar_acc_empty(a), 8);   // the epilogue warps of both CTAs
         }
         mbar_fence_init();
         abort_word = 0;
     }
     if (warp == 5) {
-        tmem_alloc(smem_u32(&tmem_slot), 512);
-        tmem_relinquish();
+        asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_slot)),
+                     "r"(2 * GN)
+                     : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
     }
     tc5_fence_before();
     __syncthreads();
+    cluster_sync();
     tc5_fence_after();
     const uint32_t tmem = tmem_slot;
     const int total = p.tiles_m * p.tiles_n, ksteps = p.inner / GK;
-    // tile t of this CTA: consecutive tiles share the row block (its 128 x inner slice of A stays in L2)
+    const int first = blockIdx.x >> 1, stride = gridDim.x >> 1;
+    // consecutive tiles share the row block (its 256 x inner slice of A stays in L2)
 
     if (warp == 4) {
         if (lane == 0) {
             tma_prefetch_desc(&map_a);
             tma_prefetch_desc(&map_b);
             int fill = 0;
-            for (int tile = blockIdx.x; tile < total; tile += gridDim.x) {
-                const int m0 = (tile / p.tiles_n) * GM, n0 = (tile % p.tiles_n) * GN;
+            for (int tile = first; tile < total; tile += stride) {
+                const int m0 = (tile / p.tiles_n) * 2 * GM + (int)rank * GM, n0 = (tile % p.tiles_n) * GN + (int)rank * (GN / 2);
                 bool ok = true;
                 for (int k = 0; k < ksteps; k++, fill++) {
-                    const int s = fill % G_STAGES, use = fill / G_STAGES;
+                    const int s = fill % ST, use = fill / ST;
                     if (use > 0 && !mbar_wait(bar_empty(s), (use - 1) & 1, &abort_word)) {
                         ok = false;
                         break;
                     }
-                    const uint32_t dst = base + s * G_STAGE;
-                    mbar_arrive_expect_tx(bar_full(s), G_STAGE);
-                    tma_load_2d(dst, &map_a, bar_full(s), k * GK, m0);
-                    tma_load_2d(dst + G_A_BYTES, &map_b, bar_full(s), k * GK, n0);
+                    const uint32_t dst = base + s * Cfg::STAGE, bar = map_to_rank(bar_full(s), 0);
+                    if (rank == 0) mbar_arrive_expect_tx(bar_full(s), 2 * Cfg::STAGE);
+                    tma_load_2d_pair(dst, &map_a, bar, k * GK, m0);
+                    tma_load_2d_pair(dst + G_A_BYTES, &map_b, bar, k * GK, n0);
                 }
                 if (!ok) break;
             }
@@ -110,34 +189,34 @@ out_proj_gate_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
     } else if (warp == 5) {
         // The whole warp walks the loop and one elected lane issues (descriptor arithmetic stays
         // in the uniform datapath; inside a one-lane branch it would be per-thread data).
-        {
+        if (rank == 0) {
             const bool leader = elect_one();
-            constexpr uint32_t idesc = mma_idesc(GM, GN, 1, 0);
+            constexpr uint32_t idesc = mma_idesc(2 * GM, GN, 1, 0);
             const uint64_t a_proto = smem_desc_sw128(base, 16, 1024), b_proto = smem_desc_sw128(base + G_A_BYTES, 16, 1024);
             const uint32_t a_lo0 = (uint32_t)a_proto, hi = (uint32_t)(a_proto >> 32), b_lo0 = (uint32_t)b_proto;
             int fill = 0, local = 0;
-            for (int tile = blockIdx.x; tile < total; tile += gridDim.x, local++) {
+            for (int tile = first; tile < total; tile += stride, local++) {
                 const int acc = local & 1;
-                bool ok = local < 2 || mbar_wait_converged(bar_acc_empty(acc), ((local >> 1) - 1) & 1, &abort_word);
+                bool ok = local < 2 || mbar_wait_cluster(bar_acc_empty(acc), ((local >> 1) - 1) & 1, &abort_word);
                 tc5_fence_after();
                 for (int k = 0; ok && k < ksteps; k++, fill++) {
-                    const int s = fill % G_STAGES;
-                    if (!mbar_wait_converged(bar_full(s), (fill / G_STAGES) & 1, &abort_word)) {
+                    const int s = fill % ST;
+                    if (!mbar_wait_cluster(bar_full(s), (fill / ST) & 1, &abort_word)) {
                         ok = false;
                         break;
                     }
                     tc5_fence_after();
-                    const uint32_t a_lo = a_lo0 + s * (G_STAGE >> 4), b_lo = b_lo0 + s * (G_STAGE >> 4);
+                    const uint32_t a_lo = a_lo0 + s * (Cfg::STAGE >> 4), b_lo = b_lo0 + s * (Cfg::STAGE >> 4);
                     if (leader) {
 #pragma unroll
                         for (int kk = 0; kk < GK / 16; kk++)
-                            mma_ss_words(tmem + acc * GN, a_lo + kk * 2, hi, b_lo + kk * 2, hi, idesc, (k > 0) || (kk > 0));
-                        mma_commit(bar_empty(s));
+                            mma_ss_pair(tmem + acc * GN, a_lo + kk * 2, hi, b_lo + kk * 2, hi, idesc, (k > 0) || (kk > 0));
+                        mma_commit_pair(bar_empty(s));
                     }
                     __syncwarp();
                 }
                 if (!ok) break;
-                if (leader) mma_commit(bar_acc_full(acc));
+                if (leader) mma_commit_pair(bar_acc_full(acc));
                 __syncwarp();
             }
         }
@@ -145,10 +224,10 @@ out_proj_gate_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
         // ---- epilogue: one thread per output row of the tile ----
         const uint32_t lane_base = (uint32_t)(warp * 32) << 16;
         int local = 0;
-        for (int tile = blockIdx.x; tile < total; tile += gridDim.x, local++) {
+        for (int tile = first; tile < total; tile += stride, local++) {
             const int acc = local & 1;
-            const int m0 = (tile / p.tiles_n) * GM, n0 = (tile % p.tiles_n) * GN;
-            if (!__all_sync(0xffffffffu, mbar_wait(bar_acc_full(acc), (local >> 1) & 1, &abort_word))) break;
+            const int m0 = (tile / p.tiles_n) * 2 * GM + (int)rank * GM, n0 = (tile % p.tiles_n) * GN;
+            if (!mbar_wait_cluster(bar_acc_full(acc), (local >> 1) & 1, &abort_word)) break;
             tc5_fence_after();
             const int row = m0 + tid;
             const bool live = row < p.rows;
@@ -187,7 +266,8 @@ out_proj_gate_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
                 }
             }
             tc5_fence_before();
-            mbar_arrive(bar_acc_empty(acc));
+            __syncwarp();
+            if (lane == 0) mbar_arrive_cluster(map_to_rank(bar_acc_empty(acc), 0));
         }
     }
     tc5_fence_before();
@@ -197,11 +277,13 @@ out_proj_gate_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
         if (warp == 4) __nanosleep(1000000);
         __syncthreads();
     }
+    cluster_sync();   // neither CTA leaves while the other's MMAs, commits or arrivals may still reach it
     if (warp == 5) {
         tc5_fence_after();
-        tmem_dealloc(tmem, 512);
+        asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(2 * GN) : "memory");
     }
 }
+
 
 // AdaLN of a row in the operation order of the reference's kernel (cuda/fast_primitives.cuh:50-124
 // with GATE = false; the reference builds with --fmad=false, hence the explicit roundings): thread
@@ -282,6 +364,27 @@ cudaError_t map_2d(CUtensorMap *map, const void *base, uint64_t rows, uint64_t c
     return r == CUDA_SUCCESS ? cudaSuccess : cudaErrorInvalidValue;
 }
 
+template <int GN>
+cudaError_t launch_proj(OutProjParams p, const void *a, const void *weight, unsigned sm_pairs, cudaStream_t stream) {
+    static thread_local int configured_device = -1;
+    int device = 0;
+    cudaError_t e = cudaGetDevice(&device);
+    if (e != cudaSuccess) return e;
+    if (configured_device != device) {
+        e = cudaFuncSetAttribute(out_proj_gate_kernel<GN>, cudaFuncAttributeMaxDynamicSharedMemorySize, ProjConfig<GN>::SMEM);
+        if (e != cudaSuccess) return e;
+        configured_device = device;
+    }
+    CUtensorMap map_a, map_b;
+    if ((e = map_2d(&map_a, a, (uint64_t)p.rows, (uint64_t)p.inner, GM)) != cudaSuccess) return e;
+    if ((e = map_2d(&map_b, weight, (uint64_t)p.hidden, (uint64_t)p.inner, GN / 2)) != cudaSuccess) return e;
+    p.tiles_m = (p.rows + 2 * GM - 1) / (2 * GM);
+    p.tiles_n = (p.hidden + GN - 1) / GN;
+    const unsigned total = (unsigned)(p.tiles_m * p.tiles_n);
+    out_proj_gate_kernel<GN><<<2 * (total < sm_pairs ? total : sm_pairs), G_THREADS, ProjConfig<GN>::SMEM, stream>>>(map_a, map_b, p);
+    return cudaGetLastError();
+}
+
 }  // namespace
 
 cudaError_t out_proj_gate(void *gated, const void *residual, const void *attention_heads, const void *weight,
@@ -290,19 +393,6 @@ cudaError_t out_proj_gate(void *gated, const void *residual, const void *attenti
     if (!rows || !inner || !hidden || inner % GK || hidden % 8 || gate_slot >= slots) return cudaErrorInvalidValue;
     for (const void *ptr : {(const void *)gated, residual, attention_heads, weight, modulation})
         if (!ptr || reinterpret_cast<uintptr_t>(ptr) % 16) return cudaErrorMisalignedAddress;
-    static thread_local int configured_device = -1, sms = 0;
-    int device = 0;
-    cudaError_t e = cudaGetDevice(&device);
-    if (e != cudaSuccess) return e;
-    if (configured_device != device) {
-        e = cudaFuncSetAttribute(out_proj_gate_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, G_SMEM);
-        if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
-        if (e != cudaSuccess) return e;
-        configured_device = device;
-    }
-    CUtensorMap map_a, map_b;
-    if ((e = map_2d(&map_a, attention_heads, rows, inner, GM)) != cudaSuccess) return e;
-    if ((e = map_2d(&map_b, weight, hidden, inner, GN)) != cudaSuccess) return e;
     OutProjParams p{};
     p.residual = static_cast<const __nv_bfloat16 *>(residual);
     p.modulation = static_cast<const __nv_bfloat16 *>(modulation);
@@ -313,12 +403,20 @@ cudaError_t out_proj_gate(void *gated, const void *residual, const void *attenti
     p.hidden = (int)hidden;
     p.slots = (int)slots;
     p.gate_slot = (int)gate_slot;
-    p.tiles_m = (int)((rows + GM - 1) / GM);
-    p.tiles_n = (int)((hidden + GN - 1) / GN);
-    if ((e = device_status_word(&p.status)) != cudaSuccess) return e;
-    const int total = p.tiles_m * p.tiles_n;
-    out_proj_gate_kernel<<<total < sms ? total : sms, G_THREADS, G_SMEM, stream>>>(map_a, map_b, p);
-    return cudaGetLastError();
+    cudaError_t e = device_status_word(&p.status);
+    if (e != cudaSuccess) return e;
+    static thread_local int sms_device = -1, sms = 0;
+    int device = 0;
+    if ((e = cudaGetDevice(&device)) != cudaSuccess) return e;
+    if (device != sms_device) {
+        if ((e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device)) != cudaSuccess) return e;
+        sms_device = device;
+    }
+    // 256-column tiles; 128-column ones, which ask half as much again of the fills per MMA, while even they
+    // do not fill the SM pairs once (few rows: then a call lasts as long as one tile).
+    const unsigned sm_pairs = (unsigned)sms / 2, narrow_tiles = (rows + 2 * GM - 1) / (2 * GM) * ((hidden + 127) / 128);
+    return narrow_tiles <= sm_pairs ? launch_proj<128>(p, attention_heads, weight, sm_pairs, stream)
+                                    : launch_proj<256>(p, attention_heads, weight, sm_pairs, stream);
 }
 
 cudaError_t adaln_rows(void *output, const void *input, const void *norm_weight, const void *modulation,

@@ -60,6 +60,19 @@ def test_against_the_oracle(gpu, oracle, rows, inner, hidden):
     assert gpu.device_status() == 0
 
 
+@pytest.mark.parametrize("rows,inner,hidden", [(2, 64, 136), (128, 192, 256), (256, 64, 5376), (257, 1088, 392), (2100, 64, 5376),
+                                               (4700, 128, 2312)])
+def test_tiles_of_two_ctas(gpu, oracle, rows, inner, hidden):
+    """Output tiles of 256 rows shared by two CTAs: the second one with no row or one, fewer k-steps than ring
+    slots and more, 128- and 256-column tiles with a ragged last one, several tiles per pair of CTAs."""
+    x, w, residual, norm_weight, modulation, row_map = out_proj_inputs(oracle, rows, inner, hidden, rows)
+    gated, _ = run_ours(gpu, x, w, residual, norm_weight, modulation, row_map)
+    want, _ = oracle.out_proj_gate_adaln(residual, x, w, norm_weight, modulation, modulation, row_map, SLOTS, GATE, SHIFT,
+                                         SCALE_SLOT)
+    close_to(oracle, gated, want, "gated residual")
+    assert gpu.device_status() == 0
+
+
 def test_argument_checks(gpu, oracle):
     x, w, residual, norm_weight, modulation, row_map = out_proj_inputs(oracle, 8, 64, 64, 1)
     t = [gpu.tensor(a) for a in (residual, x, w, norm_weight, modulation, modulation, row_map)]
