@@ -9,6 +9,10 @@ namespace h3b {
 
 // Address of this device's status word (0 = ok; see DeviceStatus in sm100_ptx.cuh).
 cudaError_t device_status_word(int **word);
+// Stream-ordered work memory (given back with cudaFreeAsync) from the library's pool of the current device, and
+// what that pool keeps but does not use handed back.
+cudaError_t work_alloc(void **pointer, size_t bytes, cudaStream_t stream);
+void work_trim(int device);
 
 // Output redirection for the sequence-gather fused into the attention epilogue: query row r of
 // local head h is stored to rank r / rows_per_rank, at [r % rows_per_rank][rank*local_heads + h]

@@ -537,7 +537,7 @@ cudaError_t attn_dense_tc5(void *out, const void *q, const void *k, const void *
                 // work memory, stream-ordered like the logsumexp buffer of the reference's wrapper
                 const size_t part_bytes = (size_t)splits * lq * heads * 256, lse_bytes = (size_t)splits * heads * lq * 4;
                 char *work = nullptr;
-                if ((e = cudaMallocAsync(reinterpret_cast<void **>(&work), part_bytes + lse_bytes, stream)) != cudaSuccess)
+                if ((e = work_alloc(reinterpret_cast<void **>(&work), part_bytes + lse_bytes, stream)) != cudaSuccess)
                     return e;
                 float *part_lse = reinterpret_cast<float *>(work + part_bytes);
                 e = attn_dense_tc5_pair(&mq, &mk, &mv, work, part_lse, 1, lq, lk, heads, kv_heads, scale, status,
@@ -660,7 +660,7 @@ cudaError_t attn_sparse_tc5(void *out, const void *q, const void *k, const void 
     unsigned char *work = nullptr;
     const size_t marks = ((size_t)tiles * heads + 255) / 256 * 256;
     const size_t work_bytes = 256 + 2 * marks;
-    if ((e = cudaMallocAsync(reinterpret_cast<void **>(&work), work_bytes, stream)) != cudaSuccess) return e;
+    if ((e = work_alloc(reinterpret_cast<void **>(&work), work_bytes, stream)) != cudaSuccess) return e;
     e = cudaMemsetAsync(work, 0, 256, stream);
     if (e == cudaSuccess)
         e = attn_sparse_t_launch(&mq64, &mk, &mv, out, lse, indices, counts, sizes, tiles, heads,

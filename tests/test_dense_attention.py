@@ -196,6 +196,36 @@ def test_causal_and_f16_at_tile_edges(gpu, oracle, L, shift):
     assert gpu.device_status() == 0
 
 
+def test_work_memory_is_kept_for_the_next_call_and_given_back(gpu, oracle):
+    """The work memory of a call stays with the library when its stream has been waited for, so that the next call
+    need not map it again, and goes when a context is freed. Two streams at once get memory of their own."""
+    import ctypes as C
+    from h3_omni_b200 import native
+    rt = native._cudart()
+
+    def free_bytes():
+        free, total = C.c_size_t(), C.c_size_t()
+        assert rt.cudaDeviceSynchronize() == 0 and rt.cudaMemGetInfo(C.byref(free), C.byref(total)) == 0
+        return free.value
+
+    other = native.Native()
+    nq, nk, heads = 200, 4500, 8
+    q, k, v = (oracle.normal_bf16((n, heads, 128), 90 + n + i) for i, n in enumerate((nq, nk, nk)))
+    outs = []
+    for _ in range(2):
+        for ctx in (gpu, other):
+            ty = ctx.empty_bf16(q.size)
+            ctx.call("cross_attention_bf16", ty, 0, ctx.tensor(q), 0, ctx.tensor(k), ctx.tensor(v), 0, nq, nk, heads)
+            outs.append((ctx, ty))
+    got = [ctx.read(ty, q.shape) for ctx, ty in outs]
+    assert all(np.array_equal(got[0], x) for x in got[1:])
+    for t in list(other.owned):
+        other.free(t)
+    before = free_bytes()
+    other.close()
+    assert free_bytes() >= before + (2 << 20)
+
+
 @pytest.mark.parametrize("column", [0, 2, 66])
 def test_not_a_number_in_a_key_reaches_its_rows(gpu, oracle, column):
     """A NaN key makes every row that attends it NaN, whichever unit takes the exponential of its column."""
