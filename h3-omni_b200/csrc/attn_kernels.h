@@ -58,21 +58,45 @@ cudaError_t attn_sparse_tc5(void *out, const void *q, const void *k, const void 
                             const int *indices, const int *counts, const int *sizes,
                             unsigned tiles, unsigned heads, cudaStream_t stream);
 
-// The persistent block-sparse kernel with the keys on the MMA's M axis (attn_sparse_t.cu), behind a
-// pre-pass that assigns every pair of adjacent query tiles to it or to the pair-walk kernel.
-// mq has a 64-row box; `ticket` (one zeroed word), `redo` and `elsewhere` ([heads][tiles] bytes
-// each) are work memory the caller provides on `stream`. After the launch redo marks the tiles the
-// pair-walk kernel has to compute: those assigned to it, and those whose row sums left the safe
-// exponent range here. assign: -1 by list overlap, 0 all here, 1 all to the pair walk.
-cudaError_t attn_sparse_t_launch(const ::CUtensorMap_st *mq, const ::CUtensorMap_st *mk,
-                                 const ::CUtensorMap_st *mv, void *out, float *lse, const int *indices,
-                                 const int *counts, const int *sizes, unsigned tiles, unsigned heads,
-                                 unsigned *ticket, unsigned char *redo, unsigned char *elsewhere, int assign,
-                                 bool force_redo, int *status, cudaStream_t stream);
-// 0 (default): pairs of query tiles whose lists mostly coincide go to the pair-walk kernel, the
-// others to the persistent kernel, whose out-of-range tiles are recomputed by the pair walk;
-// 1: pair-walk kernel only; 2: persistent kernel for everything, then every tile recomputed;
-// 3: persistent kernel for everything.
+// Work memory of a block-sparse call.
+struct SparseWork {
+    enum { TICKET_SINGLE, TICKET_PAIR, LONG, REDO, COUNTERS = 64 };
+    unsigned *counters;      // [COUNTERS]: next tickets, lengths of the lists below (zero at the start)
+    unsigned *head_sums;     // per head: list entries, and entries left when each pair of tiles joins its two lists
+                             // (zero at the start)
+    unsigned *marks;         // a bit per query tile: is on the redo list (zero at the start)
+    unsigned *redo;          // tiles (head * tiles + tile) whose row sums left the exponent range a kernel covers
+    unsigned *long_pairs;    // pairs (head * pairs + pair) with lists so long that the pair kernel starts with them
+    int assign;              // -1: every head to the kernel that its sums say; 0 / 1: all to the single / pair kernel
+    static size_t zeroed(unsigned tiles, unsigned heads) {
+        return 4 * (COUNTERS + 2 * (size_t)heads + ((size_t)tiles * heads + 31) / 32);
+    }
+    static size_t bytes(unsigned tiles, unsigned heads) {
+        return zeroed(tiles, heads) + 4 * heads * ((size_t)tiles + (tiles + 1) / 2);
+    }
+    SparseWork() = default;
+    SparseWork(void *memory, unsigned tiles, unsigned heads, int assign)
+        : counters(static_cast<unsigned *>(memory)), head_sums(counters + COUNTERS), marks(head_sums + 2 * (size_t)heads),
+          redo(counters + zeroed(tiles, heads) / 4), long_pairs(redo + (size_t)tiles * heads), assign(assign) {}
+};
+// Zeroes what has to be zero and takes the sums by which the two kernels below share the heads.
+cudaError_t attn_sparse_assign(const int *indices, const int *counts, unsigned tiles, unsigned heads,
+                               const SparseWork &work, cudaStream_t stream);
+// The persistent block-sparse kernels: every query tile walks its own list, keys on the MMA's M axis
+// (attn_sparse_t.cu; mq has a 64-row box); a pair of adjacent query tiles walks the union of its lists
+// (attn_sparse_pair.cu). Both put the tiles they could not do on the redo list (all of them with force_redo).
+cudaError_t attn_sparse_t_launch(const ::CUtensorMap_st *mq, const ::CUtensorMap_st *mk, const ::CUtensorMap_st *mv,
+                                 void *out, float *lse, const int *indices, const int *counts, const int *sizes,
+                                 unsigned tiles, unsigned heads, const SparseWork &work, bool force_redo, int *status,
+                                 cudaStream_t stream);
+cudaError_t attn_sparse_pair_launch(const ::CUtensorMap_st *mk, const ::CUtensorMap_st *mv, const void *q, void *out,
+                                    float *lse, const int *indices, const int *counts, const int *sizes,
+                                    unsigned tiles, unsigned heads, const SparseWork &work, bool force_redo, int *status,
+                                    cudaStream_t stream);
+// 0 (default): heads whose neighbouring lists overlap enough go to the pair kernel, the others to the one that
+// walks single lists, and the tiles these could not do to the running-maximum kernel of attn_tc5.cu; 1: that
+// kernel only, a CTA per pair of tiles; 2: single lists for everything, then every tile recomputed; 3: single
+// lists for everything.
 void attn_sparse_set_mode(int mode);
 
 // Warp-level mma.sync kernel (attn_mma.cu): causal / GQA bf16 D=128 and fp16 D=64.

@@ -16,8 +16,8 @@
 // reference is ONE value per query tile, the largest score of the tile's first step; any
 // reference gives the exact softmax as long as nothing over- or underflows, and the row sums
 // l[q] are kept per thread and reduced once per query tile. A query row whose sum leaves
-// [2^-60, 2^100) (or is not finite) marks its tile in `redo`, and the launcher then
-// recomputes marked tiles with the per-row online-softmax kernel of attn_tc5.cu. With
+// [2^-60, 2^100) (or is not finite) puts its tile on the `redo` list, and the launcher then
+// recomputes listed tiles with the per-row online-softmax kernel of attn_tc5.cu. With
 // attention logits inside about [-28, +69] nats of the first step's maximum nothing is marked.
 //
 // Persistent kernel, one CTA per SM, 16 warps:
@@ -31,8 +31,8 @@
 // Every wait is bounded and ends in the device status word.
 #include <cuda.h>
 
-#include "attn_kernels.h"
 #include "sm100_ptx.cuh"
+#include "sparse_heads.cuh"
 
 namespace h3b {
 namespace {
@@ -75,9 +75,7 @@ struct SparseTParams {
     const int *indices, *counts, *sizes;
     __nv_bfloat16 *out;
     float *lse;
-    unsigned *ticket;          // zero at launch
-    unsigned char *redo;       // [heads][tiles], written for every item this kernel computes
-    const unsigned char *elsewhere;   // [heads][tiles]: tiles left to the pair-walk kernel (skipped here)
+    SparseWork work;
     int *status;
     int tiles, heads, force_redo;
     float scale_log2;
@@ -201,7 +199,6 @@ attn_sparse_t_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
     __syncthreads();
     tc5_fence_after();
     const uint32_t tmem = tmem_slot;
-    const int total_items = p.tiles * p.heads;
 
     // Reads item `i`'s descriptor (waits until the scheduler has published it).
     auto fetch = [&](int i, Item &it) -> bool {
@@ -223,27 +220,31 @@ attn_sparse_t_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
         warpgroup_reg_dec<80>();
         if (warp == 10) {
             // ------------------------------ scheduler ------------------------------
+            unsigned head_nth = 0xffffffffu;
+            int head = -1;
             for (int i = 0;; i++) {
                 const int b = i & 1;
                 bool ok = true;
                 if (i >= 2) ok = mbar_wait_warp(bar_item_free(b), ((i >> 1) - 1) & 1, &abort_word);
                 if (!ok) break;
                 unsigned ticket = 0;
-                if (lane == 0) ticket = atomicAdd(p.ticket, 1u);
+                if (lane == 0) ticket = atomicAdd(p.work.counters + SparseWork::TICKET_SINGLE, 1u);
                 ticket = __shfl_sync(0xffffffffu, ticket, 0);
-                if (ticket >= (unsigned)total_items) {
+                // tickets run over this kernel's heads in order
+                const unsigned nth = ticket / (unsigned)p.tiles;
+                if (nth != head_nth) {
+                    head_nth = nth;
+                    head = nth_head(p.work, p.heads, false, nth);
+                }
+                if (head < 0) {
                     if (lane == 0) {
                         desc[b] = Item{0, 0, -1, 0};
                         mbar_arrive(bar_item_ready(b));
                     }
                     break;
                 }
-                const int head = (int)ticket / p.tiles, qt = (int)ticket % p.tiles;
+                const int qt = (int)(ticket % (unsigned)p.tiles);
                 const size_t row = (size_t)head * p.tiles + qt;
-                if (p.elsewhere[row]) {   // this tile's pair goes to the pair-walk kernel
-                    i--;
-                    continue;
-                }
                 int count = p.counts[row];
                 bool bad = count < 0 || count > p.tiles;
                 count = max(0, min(count, p.tiles));
@@ -491,7 +492,8 @@ attn_sparse_t_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
             // linv and bad_rows complete (an mbarrier, not bar.sync: a wait here must stay bounded)
             mbar_arrive(bar_epi);
             if (!mbar_wait_uniform(bar_epi, (epi_phase++) & 1, &abort_word)) break;
-            if (d == 0) p.redo[(size_t)it.head * p.tiles + it.qt] = (bad_rows[0] | bad_rows[1] | p.force_redo) ? 1 : 0;
+            if (d == 0 && (bad_rows[0] | bad_rows[1] | p.force_redo))
+                p.work.redo[atomicAdd(p.work.counters + SparseWork::REDO, 1u)] = (unsigned)(it.head * p.tiles + it.qt);
             __nv_bfloat16 *dst = p.out + out_row0 * 128 + d;
 #pragma unroll
             for (int c = 0; c < 4; c++) {
@@ -661,54 +663,6 @@ attn_sparse_t_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
     }
 }
 
-// Which kernel takes which pair of adjacent query tiles. The pair-walk kernel multiplies both
-// tiles by every KV tile of the UNION of their lists with M = 128 MMAs that read less shared
-// memory per multiply-add; this kernel multiplies each tile by its own list only. Measured cost:
-// about 990 cycles per union tile there, 692 cycles per list entry here, so a pair goes to the
-// pair walk when |A u B| < 0.7 (|A| + |B|) - lists that mostly coincide, as neighbouring cubes of
-// real video tend to produce - and stays here otherwise (also when the union is longer than 256
-// tiles). One warp per pair; both lists ascending.
-__global__ void __launch_bounds__(256)
-pair_choice_kernel(const int *__restrict__ indices, const int *__restrict__ counts, unsigned char *elsewhere,
-                   unsigned char *redo, int tiles, int heads, int force) {
-    __shared__ uint32_t bits[8][128];
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int pairs = (tiles + 1) / 2;
-    const int pair = blockIdx.x * 8 + warp, head = blockIdx.y;
-    if (pair >= pairs) return;
-    const int qa = 2 * pair, qb = qa + 1;
-    const size_t row = (size_t)head * tiles + qa;
-    int choice = 0;
-    if (force >= 0) {
-        choice = force;
-    } else if (qb < tiles) {
-        const int na = max(0, min(counts[row], tiles)), nb = max(0, min(counts[row + 1], tiles));
-        for (int w = lane; w < 128; w += 32) bits[warp][w] = 0u;
-        __syncwarp();
-        for (int i = lane; i < na; i += 32) {
-            const int kt = indices[row * tiles + i];
-            if (kt >= 0 && kt < tiles) atomicOr(&bits[warp][kt >> 5], 1u << (kt & 31));
-        }
-        __syncwarp();
-        int common = 0;
-        for (int i = lane; i < nb; i += 32) {
-            const int kt = indices[(row + 1) * tiles + i];
-            if (kt >= 0 && kt < tiles) common += (bits[warp][kt >> 5] >> (kt & 31)) & 1u;
-        }
-        common = __reduce_add_sync(0xffffffffu, common);
-        // Long lists stay with the persistent kernel whatever their overlap: there they are one
-        // ticket among thousands, while a pair-walk CTA walks its whole union alone (the prefix
-        // tiles of a video - every query tile attends all 905 KV tiles - would leave 96 CTAs
-        // running for a millisecond after everything else has finished).
-        const int joined = na + nb - common;
-        choice = (10 * joined < 7 * (na + nb) && joined <= 256) ? 1 : 0;
-    }
-    if (lane == 0) {
-        elsewhere[row] = redo[row] = (unsigned char)choice;
-        if (qb < tiles) elsewhere[row + 1] = redo[row + 1] = (unsigned char)choice;
-    }
-}
-
 }  // namespace
 
 #ifdef H3B_TRACE
@@ -719,8 +673,7 @@ extern "C" cudaError_t h3b_debug_sparse_trace(long long *host64) {
 
 cudaError_t attn_sparse_t_launch(const CUtensorMap_st *mq, const CUtensorMap_st *mk, const CUtensorMap_st *mv,
                                  void *out, float *lse, const int *indices, const int *counts, const int *sizes,
-                                 unsigned tiles, unsigned heads, unsigned *ticket, unsigned char *redo,
-                                 unsigned char *elsewhere, int assign, bool force_redo, int *status,
+                                 unsigned tiles, unsigned heads, const SparseWork &work, bool force_redo, int *status,
                                  cudaStream_t stream) {
     static thread_local int configured_device = -1, sms = 0;
     int device = 0;
@@ -738,18 +691,12 @@ cudaError_t attn_sparse_t_launch(const CUtensorMap_st *mq, const CUtensorMap_st 
     p.sizes = sizes;
     p.out = static_cast<__nv_bfloat16 *>(out);
     p.lse = lse;
-    p.ticket = ticket;
-    p.redo = redo;
-    p.elsewhere = elsewhere;
+    p.work = work;
     p.status = status;
     p.tiles = (int)tiles;
     p.heads = (int)heads;
     p.force_redo = force_redo ? 1 : 0;
     p.scale_log2 = 0.08838834764831845f * 1.4426950408889634f;   // 1/sqrt(128), fixed by the reference kernel
-    // assign: -1 = by list overlap, 0 = every pair to this kernel, 1 = every pair to the pair walk
-    pair_choice_kernel<<<dim3(((tiles + 1) / 2 + 7) / 8, heads), 256, 0, stream>>>(indices, counts, elsewhere, redo,
-                                                                                  (int)tiles, (int)heads, assign);
-    if ((e = cudaGetLastError()) != cudaSuccess) return e;
     const unsigned items = tiles * heads;
     const unsigned grid = items < (unsigned)sms ? items : (unsigned)sms;   // one persistent CTA per SM
     attn_sparse_t_kernel<<<grid, ST_THREADS, ST_SMEM, stream>>>(*mq, *mk, *mv, p);

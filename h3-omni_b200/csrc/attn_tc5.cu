@@ -15,10 +15,9 @@
 //   (cuda/flash3_attention.cu:18-94 in the reference).
 // SPARSE (BN = 64): head-major tiled [H][tiles*64][128] tensors; a CTA pairs two adjacent
 //   64-row query tiles and walks the sorted union of their selected KV tiles, masking each
-//   half against its own list and every KV tile against its valid length. (Two gathered KV
-//   tiles per step, N = 128, was tried because an N = 64 MMA reaches only two thirds of the
-//   tensor rate; it lost more by giving up the double-buffered S than it gained.) Replaces
-//   fwd_attend_ker<128> (cuda/vendor/vsa_hopper_forward.cuh:68-270) behind h3_vsa_hopper.
+//   half against its own list and every KV tile against its valid length. h3_vsa_hopper runs it on the
+//   query tiles that attn_sparse_pair.cu marks (row sums outside the range one exponent reference
+//   per row covers), one tile per CTA.
 #include <cuda.h>
 
 #include <algorithm>
@@ -45,7 +44,8 @@ struct Tc5Params {
     __nv_bfloat16 *out;
     float *lse;
     const int *indices, *counts, *sizes;
-    const unsigned char *redo;   // sparse: when set, only query tiles marked here are computed
+    // sparse recomputation: when set, the *redo_count query tiles (head * tiles + tile) listed here
+    const unsigned *redo, *redo_count;
     int tiles;
     int *status;
 };
@@ -89,16 +89,24 @@ attn_tc5_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
     auto bar_p_full = [&](int s) { return bar0 + 8u * (1 + 4 * ST + SB + s); };
     const uint32_t bar_pv_done = bar0 + 8u * (1 + 4 * ST + 2 * SB);
 
-    const int head = blockIdx.y;
     const int batch = blockIdx.z;
+    // Recomputation: a CTA takes listed query tiles one after the other (rows 64-127 idle, so that a tile
+    // meets no keys but its own). Few or none are listed: it leaves before anything is set up.
+    const bool single = SPARSE && p.redo;
+    const unsigned redo_count = single ? min(*p.redo_count, (unsigned)(p.tiles * p.heads)) : 1u;
+    if (single && blockIdx.x >= redo_count) return;
+    uint32_t tmem = 0;
+    for (unsigned turn = single ? blockIdx.x : 0u; turn < redo_count; turn += single ? gridDim.x : 1u) {
+    const bool first_turn = !single || turn == blockIdx.x;
+    const int head = single ? (int)(p.redo[turn] / (unsigned)p.tiles) : (int)blockIdx.y;
     const int kv_head = SPARSE ? head : head / (p.heads / p.kv_heads);
-    const int q_row0 = blockIdx.x * BM;  // dense: token row; sparse: padded tiled row
-
-    if (SPARSE && p.redo) {
-        // recomputation pass: leave at once unless one of this CTA's two query tiles is marked
-        const size_t first = (size_t)head * p.tiles + blockIdx.x * 2;
-        const bool second = blockIdx.x * 2 + 1 < p.tiles;
-        if (!p.redo[first] && !(second && p.redo[first + 1])) return;
+    // dense: token row; sparse: padded tiled row
+    const int q_row0 = single ? (int)(p.redo[turn] % (unsigned)p.tiles) * 64 : (int)blockIdx.x * BM;
+    if (!first_turn) {
+        __syncthreads();   // every wait of the turn before is over, and every commit has arrived (see the issuer)
+        if (abort_word) break;
+        if (tid == 0)
+            for (int i = 0; i < 1 + 4 * ST + 2 * SB + 1; i++) mbar_inval(bar0 + 8u * i);
     }
 
     if (tid == 0) {
@@ -115,26 +123,26 @@ attn_tc5_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
         }
         mbar_init(bar_pv_done, 1);
         mbar_fence_init();
-        abort_word = 0;
+        if (first_turn) abort_word = 0;
         union_count = 0;
     }
     if (SPARSE && tid < 128) {
         bits_a[tid] = 0;
         bits_b[tid] = 0;
     }
-    if (warp == 5) {
+    if (warp == 5 && first_turn) {
         tmem_alloc(smem_u32(&tmem_slot), TMEM_COLS);
         tmem_relinquish();
     }
     tc5_fence_before();
     __syncthreads();
     tc5_fence_after();
-    const uint32_t tmem = tmem_slot;
+    tmem = tmem_slot;
 
     int n_tiles;  // KV tiles this CTA walks
     if (SPARSE) {
         // Bitmaps of the KV tiles selected by query tile A (rows 0-63) and B (rows 64-127).
-        const int qa = blockIdx.x * 2, qb = qa + 1;
+        const int qa = q_row0 / 64, qb = single ? p.tiles : qa + 1;
         const size_t row_a = (size_t)head * p.tiles + qa;
         const int raw_a = p.counts[row_a], raw_b = qb < p.tiles ? p.counts[row_a + 1] : 0;
         // a count outside [0, tiles] is refused like a bad index; the list is clamped
@@ -278,13 +286,26 @@ attn_tc5_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
                 mma_commit(bar_pv_done);
                 if (SB == 1 && j + 1 < n_tiles && !issue_qk(j + 1)) break;
             }
+            // the barriers are set up anew for the next turn: let the last commit to each slot arrive
+            for (int s = 0; single && s < ST && s < n_tiles; s++) {
+                const uint32_t parity = ((n_tiles - 1 - s) / ST) & 1;
+                if (!mbar_wait(bar_k_empty(s), parity, &abort_word) || !mbar_wait(bar_v_empty(s), parity, &abort_word)) break;
+            }
         }
     } else {
         // ------------------------------ online softmax ------------------------------
         const int r = tid;  // query row inside the tile == TMEM lane
         const uint32_t lane_base = (uint32_t)(warp * 32) << 16;
         const int half = r >> 6;
-        float m_ref = -INFINITY, l = 0.0f;
+        // The sum of a sparse row is kept in two parts, by the parity of the row's own list position:
+        // the order attn_sparse_pair_kernel adds in, so that a pair of equal lists gives equal bits.
+        float m_ref = -INFINITY, l = 0.0f, l_odd = 0.0f;
+        bool odd = false;
+        auto add_to_sum = [&](float x) {
+            if (SPARSE && odd) l_odd += x;
+            else l += x;
+            odd = !odd;
+        };
         bool alive = true;
         for (int j = 0; j < n_tiles; j++) {
             int kt, flags;
@@ -320,6 +341,7 @@ attn_tc5_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
                 const float alpha = grow ? fast_exp2((m_ref - m_new) * p.scale_log2) : 1.0f;
                 if (grow) m_ref = m_new;
                 l *= alpha;
+                l_odd *= alpha;
                 if (j > 0) {
                     alive = __all_sync(0xffffffffu,
                                        mbar_wait(bar_pv_done, (j - 1) & 1, &abort_word));
@@ -341,9 +363,9 @@ attn_tc5_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
             }
             const float neg = (m_ref == -INFINITY) ? 0.0f : -m_ref * p.scale_log2;
             if (nvalid >= BN) {
-                l += exp_store_full<BN>(s_addr, s_addr, p.scale_log2, neg);
+                add_to_sum(exp_store_full<BN, SPARSE>(s_addr, s_addr, p.scale_log2, neg));
             } else if (nvalid > 0) {
-                l += exp_store_masked<BN>(s_addr, s_addr, p.scale_log2, neg, nvalid);
+                add_to_sum(exp_store_masked<BN, SPARSE>(s_addr, s_addr, p.scale_log2, neg, nvalid));
             } else {
                 store_zero_p<BN>(s_addr);  // this half of the pair did not select the tile
             }
@@ -364,7 +386,7 @@ attn_tc5_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
         if (SPARSE && alive && n_tiles == 0) {
             // neither query tile selected anything: defined result, zero rows
             const int padded = q_row0 + r;
-            if (padded < p.tiles * 64) {
+            if (padded < p.tiles * 64 && !(single && r >= 64)) {
                 uint4 *d4 = reinterpret_cast<uint4 *>(p.out + ((size_t)head * p.tiles * 64 + padded) * HD);
 #pragma unroll
                 for (int i = 0; i < HD / 8; i++) d4[i] = make_uint4(0u, 0u, 0u, 0u);
@@ -373,12 +395,13 @@ attn_tc5_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
         }
         if (alive && n_tiles > 0) {
             tc5_fence_after();
+            l += l_odd;
             const float inv = l > 0.0f ? 1.0f / l : 0.0f;   // a half with an empty list: zero rows
             bool store;
             __nv_bfloat16 *dst;
             if (SPARSE) {
                 const int padded = q_row0 + r;
-                store = padded < p.tiles * 64;
+                store = padded < p.tiles * 64 && !(single && r >= 64);
                 dst = p.out + ((size_t)head * p.tiles * 64 + padded) * HD;
                 if (store && p.lse)
                     p.lse[(size_t)head * p.tiles * 64 + padded] =
@@ -414,6 +437,9 @@ attn_tc5_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
                 }
             }
         }
+    }
+
+    tc5_fence_before();
     }
 
     // ---------------------------------- teardown ----------------------------------
@@ -654,24 +680,25 @@ cudaError_t attn_sparse_tc5(void *out, const void *q, const void *k, const void 
     dim3 grid((tiles + 1) / 2, heads, 1);
     const int mode = g_sparse_mode;
     if (mode == 1) return launch<64, true>(mq, mk, mv, p, grid, stream);
-    // Work memory of the persistent kernel, stream-ordered like the logsumexp buffer the
-    // reference's wrapper allocates per call (cuda/h3_gpu_cuda.cu:1115-1127): one ticket word
-    // and two marks per query tile.
-    unsigned char *work = nullptr;
-    const size_t marks = ((size_t)tiles * heads + 255) / 256 * 256;
-    const size_t work_bytes = 256 + 2 * marks;
-    if ((e = work_alloc(reinterpret_cast<void **>(&work), work_bytes, stream)) != cudaSuccess) return e;
-    e = cudaMemsetAsync(work, 0, 256, stream);
+    // Work memory, stream-ordered like the logsumexp buffer the reference's wrapper allocates per call
+    // (cuda/h3_gpu_cuda.cu:1115-1127).
+    void *memory = nullptr;
+    if ((e = work_alloc(&memory, SparseWork::bytes(tiles, heads), stream)) != cudaSuccess) return e;
+    const SparseWork work(memory, tiles, heads, mode == 0 ? -1 : 0);
+    e = attn_sparse_assign(indices, counts, tiles, heads, work, stream);
+    if (e == cudaSuccess && mode == 0)
+        e = attn_sparse_pair_launch(&mk, &mv, q, out, lse, indices, counts, sizes, tiles, heads, work, false, status, stream);
     if (e == cudaSuccess)
-        e = attn_sparse_t_launch(&mq64, &mk, &mv, out, lse, indices, counts, sizes, tiles, heads,
-                                 reinterpret_cast<unsigned *>(work), work + 256, work + 256 + marks,
-                                 mode == 0 ? -1 : 0, mode == 2, status, stream);
+        e = attn_sparse_t_launch(&mq64, &mk, &mv, out, lse, indices, counts, sizes, tiles, heads, work, mode == 2, status,
+                                 stream);
     if (e == cudaSuccess) {
-        // marked tiles (row sums outside the safe exponent range) are recomputed with per-row maxima
-        p.redo = work + 256;
-        e = launch<64, true>(mq, mk, mv, p, grid, stream);
+        // Listed tiles (row sums outside the safe exponent range) are recomputed with running maxima. Hardly
+        // ever is there one, so the launch is small: with a CTA per tile it took 90 to 120 us to find none.
+        p.redo = work.redo;
+        p.redo_count = work.counters + SparseWork::REDO;
+        e = launch<64, true>(mq, mk, mv, p, dim3(tiles * heads < 296u ? tiles * heads : 296u, 1, 1), stream);
     }
-    const cudaError_t freed = cudaFreeAsync(work, stream);
+    const cudaError_t freed = cudaFreeAsync(memory, stream);
     return e != cudaSuccess ? e : freed;
 }
 

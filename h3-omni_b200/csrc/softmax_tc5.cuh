@@ -74,8 +74,15 @@ __device__ __forceinline__ float row_max_masked(uint32_t s_addr, int nvalid) {
     }
     return mx;
 }
+// What a row sum adds for a packed pair of weights: with ROUNDED the bf16 values that the PV product uses,
+// so that numerator and denominator agree.
+template <bool ROUNDED>
+__device__ __forceinline__ float2 summand(float2 p, uint32_t packed) {
+    return ROUNDED ? make_float2(__uint_as_float(packed << 16), __uint_as_float(packed & 0xffff0000u)) : p;
+}
 // p = exp2(s * scale_log2 + neg) for 32 columns, packed pairwise to bf16; partial row sums
 // accumulate in two float2 chains (packed f32x2 arithmetic halves the FMA-pipe work).
+template <bool ROUNDED = false>
 __device__ __forceinline__ void exp_chunk(const uint32_t (&v)[32], uint32_t (&packed)[16],
                                           float2 scale2, float2 neg2, float2 &sum0, float2 &sum1) {
 #pragma unroll
@@ -86,15 +93,15 @@ __device__ __forceinline__ void exp_chunk(const uint32_t (&v)[32], uint32_t (&pa
             make_float2(__uint_as_float(v[i + 2]), __uint_as_float(v[i + 3])), scale2, neg2);
         const float2 p0 = make_float2(fast_exp2(x0.x), fast_exp2(x0.y));
         const float2 p1 = make_float2(fast_exp2(x1.x), fast_exp2(x1.y));
-        sum0 = __fadd2_rn(sum0, p0);
-        sum1 = __fadd2_rn(sum1, p1);
         packed[i / 2] = pack_bf16(p0.x, p0.y);
         packed[i / 2 + 1] = pack_bf16(p1.x, p1.y);
+        sum0 = __fadd2_rn(sum0, summand<ROUNDED>(p0, packed[i / 2]));
+        sum1 = __fadd2_rn(sum1, summand<ROUNDED>(p1, packed[i / 2 + 1]));
     }
 }
 // Full tile: P (bf16 pairs, half the columns) goes to p_addr - over columns of S that were
 // already consumed - with the loads running one chunk ahead.
-template <int BN>
+template <int BN, bool ROUNDED>
 __device__ __forceinline__ float exp_store_full(uint32_t s_addr, uint32_t p_addr, float scale_log2,
                                                 float neg) {
     constexpr int NC = BN / 32;
@@ -106,22 +113,24 @@ __device__ __forceinline__ float exp_store_full(uint32_t s_addr, uint32_t p_addr
 #pragma unroll
     for (int c = 0; c < NC; c += 2) {
         if (c + 1 < NC) tmem_ld32(s_addr + (c + 1) * 32, b);
-        exp_chunk(a, packed, scale2, neg2, sum0, sum1);
+        exp_chunk<ROUNDED>(a, packed, scale2, neg2, sum0, sum1);
         tmem_st16(p_addr + c * 16, packed);
         if (c + 1 < NC) {
             tmem_wait_ld();
             if (c + 2 < NC) tmem_ld32(s_addr + (c + 2) * 32, a);
-            exp_chunk(b, packed, scale2, neg2, sum0, sum1);
+            exp_chunk<ROUNDED>(b, packed, scale2, neg2, sum0, sum1);
             tmem_st16(p_addr + (c + 1) * 16, packed);
             if (c + 2 < NC) tmem_wait_ld();
         }
     }
     return (sum0.x + sum0.y) + (sum1.x + sum1.y);
 }
-template <int BN>
+// The same for a tile of which only the first nvalid columns count.
+template <int BN, bool ROUNDED>
 __device__ __forceinline__ float exp_store_masked(uint32_t s_addr, uint32_t p_addr, float scale_log2,
                                                   float neg, int nvalid) {
-    float sum = 0.0f;
+    float2 sum0 = make_float2(0.f, 0.f), sum1 = make_float2(0.f, 0.f);
+    const float2 scale2 = make_float2(scale_log2, scale_log2), neg2 = make_float2(neg, neg);
 #pragma unroll
     for (int c = 0; c < BN / 32; c++) {
         uint32_t v[32], packed[16];
@@ -129,16 +138,17 @@ __device__ __forceinline__ float exp_store_masked(uint32_t s_addr, uint32_t p_ad
         tmem_wait_ld();
 #pragma unroll
         for (int i = 0; i < 32; i += 2) {
-            float p0 = fast_exp2(fmaf(__uint_as_float(v[i]), scale_log2, neg));
-            float p1 = fast_exp2(fmaf(__uint_as_float(v[i + 1]), scale_log2, neg));
-            if (c * 32 + i >= nvalid) p0 = 0.0f;
-            if (c * 32 + i + 1 >= nvalid) p1 = 0.0f;
-            sum += p0 + p1;
-            packed[i / 2] = pack_bf16(p0, p1);
+            // (a weight of zero, not a score of -inf: the caller's scale may be zero or negative)
+            const float2 x = __ffma2_rn(make_float2(__uint_as_float(v[i]), __uint_as_float(v[i + 1])), scale2, neg2);
+            const float2 p = make_float2(c * 32 + i < nvalid ? fast_exp2(x.x) : 0.0f,
+                                         c * 32 + i + 1 < nvalid ? fast_exp2(x.y) : 0.0f);
+            packed[i / 2] = pack_bf16(p.x, p.y);
+            float2 &sum = (i & 2) ? sum1 : sum0;
+            sum = __fadd2_rn(sum, summand<ROUNDED>(p, packed[i / 2]));
         }
         tmem_st16(p_addr + c * 16, packed);
     }
-    return sum;
+    return (sum0.x + sum0.y) + (sum1.x + sum1.y);
 }
 template <int BN>
 __device__ __forceinline__ void store_zero_p(uint32_t p_addr) {

@@ -401,14 +401,13 @@ int h3b_vsa_qkv_rope_bf16(h3_gpu_vsa *vsa, h3_gpu_tensor *output, const h3_gpu_t
                           const h3_gpu_tensor *gate, uint32_t rope_half, float epsilon, int grouped);
 
 /* Which kernel runs the block-sparse fine stage behind h3_vsa_hopper (process-wide; for A/B
- * measurement and tests). There are two: the persistent kernel, in which every query tile walks
- * its own list only, and the pair-walk kernel, in which a CTA takes two adjacent query tiles and
- * walks the union of their lists (per-row online softmax; cheaper per multiply-add, wasteful when
- * the two lists differ). 0 (default): a pre-pass gives every pair of tiles to the pair walk when
- * their lists mostly coincide (|A u B| < 0.7 (|A| + |B|)) and to the persistent kernel otherwise;
- * the rare tiles whose softmax sums leave the exponent range the persistent kernel covers are
- * recomputed by the pair walk. 1: pair-walk kernel only. 2: persistent kernel, then every tile
- * recomputed by the pair walk. 3: persistent kernel for every pair. */
+ * measurement and tests). There are three: the single kernel, in which every query tile walks its own
+ * list; the pair kernel, in which two adjacent query tiles walk the union of their lists (cheaper per
+ * multiply-add, wasteful when the lists differ); and the running-maximum kernel (per-row online
+ * softmax). 0 (default): a head goes to the pair kernel when joining the lists of its pairs leaves
+ * less than 75 % of their entries and to the single kernel otherwise; the rare tiles whose softmax
+ * sums leave the exponent range these two cover are recomputed with running maxima. 1: running-maximum
+ * kernel only. 2: single kernel, then every tile recomputed. 3: single kernel for every head. */
 void h3b_vsa_fine_mode(int mode);
 
 /* Top-k tile selection of video sparse attention with no device allocation at all. It has no

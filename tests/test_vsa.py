@@ -350,6 +350,47 @@ def test_vsa_fine_extreme_logits_are_recomputed(gpu, oracle):
     assert np.abs(out - want)[:, mild].max() <= 1e-2
 
 
+@pytest.mark.parametrize("tiles,heads", [(1, 1), (2, 3), (13, 24), (64, 5), (65, 3)])
+def test_vsa_fine_walk_lengths(gpu, oracle, tiles, heads):
+    """Walks of one step, of fewer and of more steps than there are score tiles and ring slots, long ones
+    (which are handed out first) among short ones, an odd last tile, more pairs than SMs, no full tile; lists of
+    neighbours once alike (pair kernel) and once not. A result is rounded to 2^-9 of itself and is a mean of
+    values with weights rounded to 2^-9 above and below the line."""
+    rng = np.random.default_rng(tiles)
+    sizes = rng.integers(1, 65, tiles).astype(np.int32)
+    q, k, v = (oracle.normal_bf16((heads, tiles * 64, 128), 60 + tiles + i) for i in range(3))
+    indices, counts = _random_lists(rng, tiles, heads)
+    for h in range(heads):
+        for t in range(tiles):
+            if (h + t // 2) % 3:   # two pairs in three are short
+                counts[h, t] = min(counts[h, t], 1 + (t + h) % 7)
+    limit = (2.0 ** -9 + 2 * 2.0 ** -9) * float(np.abs(oracle.from_bf16(v)).max())
+    for alike in (False, True):
+        if alike:
+            indices[:, 1::2], counts[:, 1::2] = indices[:, 0:tiles // 2 * 2:2], counts[:, 0:tiles // 2 * 2:2]
+        bits, _ = _fine_direct(gpu, q, k, v, indices, counts, sizes)
+        _, want, _ = oracle.vsa_fine(q, k, v, indices, counts, sizes)
+        assert np.abs(oracle.from_bf16(bits) - want).max() <= limit, alike
+
+
+def test_vsa_fine_infinite_value_stays_with_its_readers(gpu, oracle):
+    """An infinity in V reaches the query tiles that selected its tile and no others, also where the other
+    tile of the pair did."""
+    tiles, heads, poisoned = 6, 1, 3
+    sizes = np.full(tiles, 64, dtype=np.int32)
+    q, k, v = (oracle.normal_bf16((heads, tiles * 64, 128), 80 + i) for i in range(3))
+    indices = np.zeros((heads, tiles, tiles), dtype=np.int32)
+    counts = np.zeros((heads, tiles), dtype=np.int32)
+    for t in range(tiles):
+        chosen = [x for x in range(tiles) if x != poisoned] if t % 2 else list(range(tiles))   # alike: the pair kernel
+        indices[0, t, :len(chosen)], counts[0, t] = chosen, len(chosen)
+    _, want, _ = oracle.vsa_fine(q, k, v, indices, counts, sizes)
+    v[0, poisoned * 64 + 5, 7] = 0x7f80
+    out = oracle.from_bf16(_fine_direct(gpu, q, k, v, indices, counts, sizes)[0]).reshape(tiles, 64, 128)
+    assert not np.isfinite(out[0::2, :, 7]).any()
+    assert np.abs(out[1::2] - want.reshape(tiles, 64, 128)[1::2]).max() <= 1e-2
+
+
 def test_vsa_hopper_rejects_bad_lists(gpu, oracle):
     """An out-of-range tile index is refused on the device (status 2), never dereferenced."""
     tiles, heads = 4, 1
