@@ -83,91 +83,121 @@ tile_pool_kernel(PoolArgs a, const int *__restrict__ map, const int *__restrict_
 }
 
 // ---- scores + top-k selection + compression -----------------------------------------
-constexpr int CHUNK = 64;    // pooled K/V rows staged per step
-constexpr int PADDED = VD + 4;  // 16-byte aligned rows; float4 reads of 8 consecutive rows hit 32 distinct banks
+constexpr int KCHUNK = 128, KHALF = 64;   // pooled K staged per step: 128 rows x 64 dims
+constexpr int KPAD = KHALF + 4;           // rows 4 banks apart: 8 rows x 16 bytes hit 32 distinct banks
+constexpr int QPAD = VD + 4;
+constexpr int VCHUNK = 64;                // pooled V rows staged per step
+static_assert(VCHUNK * VD <= KCHUNK * KPAD, "V stage fits the K stage");
+// Floats between two score rows: float4-aligned and 4 banks apart like the rows above.
+__host__ __device__ constexpr int score_stride(int tiles) { return (tiles + 31) / 32 * 32 + 4; }
 
 // Order-preserving key of a float, the one cub's radix sort uses: larger float -> larger key.
 __device__ __forceinline__ uint32_t sort_key(float f) {
     const uint32_t u = __float_as_uint(f);
     return (u & 0x80000000u) ? ~u : (u | 0x80000000u);
 }
+__device__ __forceinline__ uint32_t tile_key(float f) { return max(sort_key(f), 1u); }   // 0 stands for "no tile"
+__device__ __forceinline__ float key_value(uint32_t k) {
+    return __uint_as_float((k & 0x80000000u) ? k ^ 0x80000000u : ~k);
+}
 
-// One CTA = 8 * QPW query tiles of one head, 8 warps; warp w owns query tiles w, w + 8, ...
-// for selection, softmax and compression. Pooled K (then V) rows stream through shared
-// memory in chunks of 32, the next chunk's global loads in flight while the current one is
-// used, so each pooled row is read from L2 once per 8 * QPW query tiles.
+// One CTA = 8 * QPW query tiles of one head, 8 warps. Pooled K (then V) rows stream through shared
+// memory, the next chunk's global loads in flight while the current one is used, so each pooled row is
+// read from L2 once per 8 * QPW query tiles.
 //   scores row = scale * fmaf-chain over d = 0..127 (ascending), one fixed order.
 //   Selection (cuda/vsa.cuh:47-76): prefix query tiles keep all tiles; video query tiles keep
 //   all prefix tiles plus the `keep` best video tiles (ties: lower index first), ascending.
 //   Compression (cuda/vsa.cuh:80-166,291-294): softmax over the whole row in the ATen lane
 //   order, then sum_k p[k] * poolv[k][:] as one fmaf chain over k ascending.
+// Both products are bound by shared-memory wavefronts unless a read feeds several FMAs: a warp covers 8 rows
+// (or 8 x 4 dims) by 4 query tiles, so that a vector read is one wavefront, broadcast to the other lanes, and
+// a thread takes 4 keys x QPW query tiles of the scores (4 + QPW wavefronts per 16 * QPW FMAs) and 4 dims x
+// QPW query tiles of the compression (4 + QPW per 4 keys and 16 * QPW FMAs).
+// 905 tiles x 24 heads: 754 us with a key row (or four dims) per lane and a bit-by-bit search, 704 with this tiling,
+// 660 with the interval search below (287 tiles x 56 heads: 231 -> 198 for the search).
 template <int QPW>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(256, 2)
 score_select_kernel(const float *__restrict__ poolq, const float *__restrict__ poolk,
                     const float *__restrict__ poolv, float *__restrict__ scores_out,
                     int *__restrict__ indices, int *__restrict__ counts,
                     float *__restrict__ compression, int tiles, int prefix, int keep, float scale) {
     constexpr int QT = 8 * QPW;
-    extern __shared__ float sm[];
-    float *row_scores = sm;                               // [QT][tiles]
-    float *stage = row_scores + (size_t)QT * tiles;       // [CHUNK][PADDED]
-    float *qrows = stage + CHUNK * PADDED;                // [QT][VD]
+    extern __shared__ __align__(16) float sm[];
+    const int stride = score_stride(tiles);
+    float *row_scores = sm;                                // [QT][stride]
+    float *stage = row_scores + (size_t)QT * stride;       // [KCHUNK][KPAD], later [VCHUNK][VD]
+    float *qrows = stage + KCHUNK * KPAD;                  // [QT][QPAD]
 
     const int head = blockIdx.y, qt0 = blockIdx.x * QT;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int nq = min(QT, tiles - qt0);
-    const float *pk = poolk + (size_t)head * tiles * VD;
+    const int in8 = lane & 7, in4 = lane >> 3;
 
     for (int i = tid; i < QT * VD; i += 256) {
-        const int qi = i / VD;
-        qrows[i] = qi < nq ? poolq[((size_t)head * tiles + qt0 + qi) * VD + (i % VD)] : 0.0f;
+        const int qi = i / VD, d = i % VD;
+        qrows[qi * QPAD + d] = qi < nq ? poolq[((size_t)head * tiles + qt0 + qi) * VD + d] : 0.0f;
     }
-    // ---- scores: thread = (key row r of the chunk, query group); 4 * QPW dot products per
-    // thread from float4 shared-memory reads (the pass is bound by shared-memory wavefronts:
-    // 4 for the key vector + 1 per broadcast query vector feed 16 * QPW FMAs) ----
+    // ---- scores: warp = 32 keys (of 128) x 4 * QPW query tiles ----
     {
-        constexpr int NQ = 4 * QPW;            // query rows per thread: group + 4 g... (QT / 4)
-        constexpr int PER_THREAD = CHUNK * VD / 256;
-        float next[PER_THREAD];   // this thread's elements of the chunk being fetched
-        auto fetch = [&](int k0) {
+        const float *pk = poolk + (size_t)head * tiles * VD;
+        const bool wide = reinterpret_cast<uintptr_t>(poolk) % 16 == 0;   // a caller's own array need not be
+        constexpr int PER_THREAD = KCHUNK * KHALF / 4 / 256;
+        float4 next[PER_THREAD];   // this thread's part of the stage being fetched
+        auto fetch = [&](int k0, int half) {
 #pragma unroll
             for (int u = 0; u < PER_THREAD; u++) {
-                const int i = tid + u * 256, r = i / VD, d = i % VD;
-                next[u] = k0 + r < tiles ? __ldg(pk + (size_t)(k0 + r) * VD + d) : 0.0f;
+                const int i = tid + u * 256, r = i / (KHALF / 4), c = i % (KHALF / 4);
+                const float *at = pk + (size_t)(k0 + r) * VD + half * KHALF + c * 4;
+                next[u] = make_float4(0.f, 0.f, 0.f, 0.f);
+                if (k0 + r < tiles)
+                    next[u] = wide ? __ldg(reinterpret_cast<const float4 *>(at))
+                                   : make_float4(__ldg(at), __ldg(at + 1), __ldg(at + 2), __ldg(at + 3));
             }
         };
-        fetch(0);
-        const int r = tid & (CHUNK - 1), group = tid / CHUNK;   // 64 key rows x 4 query groups
-        for (int k0 = 0; k0 < tiles; k0 += CHUNK) {
-            __syncthreads();   // previous chunk fully consumed
+        fetch(0, 0);
+        const int key0 = (warp >> 1) * 32 + in8, q0 = (warp & 1) * 4 * QPW + in4;
+        for (int k0 = 0; k0 < tiles; k0 += KCHUNK) {
+            float dot[4][QPW];
 #pragma unroll
-            for (int u = 0; u < PER_THREAD; u++) {
-                const int i = tid + u * 256;
-                stage[(i / VD) * PADDED + (i % VD)] = next[u];
-            }
-            __syncthreads();
-            if (k0 + CHUNK < tiles) fetch(k0 + CHUNK);
-            if (k0 + r < tiles) {
-                const float4 *kr = reinterpret_cast<const float4 *>(stage + r * PADDED);
-                float dot[NQ];
+            for (int i = 0; i < 4; i++)
 #pragma unroll
-                for (int g = 0; g < NQ; g++) dot[g] = 0.0f;
-#pragma unroll 4
-                for (int d4 = 0; d4 < VD / 4; d4++) {
-                    const float4 kv = kr[d4];
+                for (int u = 0; u < QPW; u++) dot[i][u] = 0.0f;
+#pragma unroll 1
+            for (int half = 0; half < 2; half++) {
+                __syncthreads();   // the stage is used up
 #pragma unroll
-                    for (int g = 0; g < NQ; g++) {
-                        const float4 qv = reinterpret_cast<const float4 *>(qrows + (group + 4 * g) * VD)[d4];
-                        dot[g] = fmaf(qv.x, kv.x, dot[g]);
-                        dot[g] = fmaf(qv.y, kv.y, dot[g]);
-                        dot[g] = fmaf(qv.z, kv.z, dot[g]);
-                        dot[g] = fmaf(qv.w, kv.w, dot[g]);
-                    }
+                for (int u = 0; u < PER_THREAD; u++) {
+                    const int i = tid + u * 256;
+                    *reinterpret_cast<float4 *>(stage + (i / (KHALF / 4)) * KPAD + (i % (KHALF / 4)) * 4) = next[u];
                 }
+                __syncthreads();
+                if (half == 0) fetch(k0, 1);
+                else if (k0 + KCHUNK < tiles) fetch(k0 + KCHUNK, 0);
+#pragma unroll 4
+                for (int d = 0; d < KHALF; d += 4) {
+                    float4 kv[4], qv[QPW];
 #pragma unroll
-                for (int g = 0; g < NQ; g++)
-                    if (group + 4 * g < nq) row_scores[(size_t)(group + 4 * g) * tiles + k0 + r] = scale * dot[g];
+                    for (int i = 0; i < 4; i++) kv[i] = *reinterpret_cast<const float4 *>(stage + (key0 + 8 * i) * KPAD + d);
+#pragma unroll
+                    for (int u = 0; u < QPW; u++)
+                        qv[u] = *reinterpret_cast<const float4 *>(qrows + (q0 + 4 * u) * QPAD + half * KHALF + d);
+#pragma unroll
+                    for (int i = 0; i < 4; i++)
+#pragma unroll
+                        for (int u = 0; u < QPW; u++) {
+                            dot[i][u] = fmaf(qv[u].x, kv[i].x, dot[i][u]);
+                            dot[i][u] = fmaf(qv[u].y, kv[i].y, dot[i][u]);
+                            dot[i][u] = fmaf(qv[u].z, kv[i].z, dot[i][u]);
+                            dot[i][u] = fmaf(qv[u].w, kv[i].w, dot[i][u]);
+                        }
+                }
             }
+#pragma unroll
+            for (int i = 0; i < 4; i++)
+#pragma unroll
+                for (int u = 0; u < QPW; u++)
+                    if (k0 + key0 + 8 * i < tiles && q0 + 4 * u < nq)
+                        row_scores[(size_t)(q0 + 4 * u) * stride + k0 + key0 + 8 * i] = scale * dot[i][u];
         }
     }
     __syncthreads();
@@ -178,7 +208,7 @@ score_select_kernel(const float *__restrict__ poolq, const float *__restrict__ p
         const int qi = warp + 8 * g;
         if (qi >= nq) break;
         const int qt = qt0 + qi;
-        float *mine = row_scores + (size_t)qi * tiles;
+        float *mine = row_scores + (size_t)qi * stride;
         const size_t row = (size_t)head * tiles + qt;
         if (scores_out)
             for (int j = lane; j < tiles; j += 32) scores_out[row * tiles + j] = mine[j];
@@ -187,44 +217,64 @@ score_select_kernel(const float *__restrict__ poolq, const float *__restrict__ p
             for (int j = lane; j < tiles; j += 32) dst[j] = j;
             if (lane == 0) counts[row] = tiles;
         } else {
-            // The keep-th largest key among the video tiles, found bit by bit from the top:
-            // `want` grows by a bit whenever at least `keep` keys are still >= the candidate.
-            // Counting is a compare per key and one warp reduction per bit - no shared-memory
-            // histogram, no atomics.
-            uint32_t want = 0u;
-            int greater = 0;
-            if (tiles - prefix <= 32 * 32) {
-                // up to 1024 video tiles: this lane's keys live in registers for all 33 passes
-                uint32_t key[32];
+            // The keep-th largest key among the video tiles lies in [low, high): at least `keep` keys are
+            // >= low, fewer are >= high. The interval is halved first by value, then (ties, infinities)
+            // by key, until exactly `keep` keys are >= low - about a dozen counts, where a bit-by-bit search
+            // takes 32 - or one key is left. Counting is a compare per key and one warp reduction: no
+            // shared-memory histogram, no atomics.
+            uint32_t key[32];   // up to 1024 video tiles: this lane's keys stay in registers
+            const bool in_registers = tiles - prefix <= 32 * 32;
+            const int groups = (tiles - prefix + 255) / 256;   // of eight keys per lane
+            if (in_registers) {
 #pragma unroll
                 for (int i = 0; i < 32; i++) {
                     const int j = prefix + lane + 32 * i;
-                    key[i] = j < tiles ? sort_key(mine[j]) : 0u;   // 0 is below every real key
+                    if (i / 8 < groups) key[i] = j < tiles ? tile_key(mine[j]) : 0u;   // 0 is below every real key
                 }
-                for (int bit = 31; bit >= 0; bit--) {
-                    const uint32_t candidate = want | (1u << bit);
-                    int count = 0;
-#pragma unroll
-                    for (int i = 0; i < 32; i++) count += key[i] >= candidate;
-                    if (__reduce_add_sync(0xffffffffu, count) >= keep) want = candidate;
-                }
-#pragma unroll
-                for (int i = 0; i < 32; i++) greater += key[i] > want;
-                greater = __reduce_add_sync(0xffffffffu, greater);
-            } else {
-                for (int bit = 31; bit >= 0; bit--) {
-                    const uint32_t candidate = want | (1u << bit);
-                    int count = 0;
-                    for (int j = prefix + lane; j < tiles; j += 32) count += sort_key(mine[j]) >= candidate;
-                    if (__reduce_add_sync(0xffffffffu, count) >= keep) want = candidate;
-                }
-                for (int j = prefix + lane; j < tiles; j += 32) greater += sort_key(mine[j]) > want;
-                greater = __reduce_add_sync(0xffffffffu, greater);
             }
+            auto each_key = [&](auto visit) {
+                if (in_registers) {
+#pragma unroll
+                    for (int i = 0; i < 32; i++)
+                        if (i / 8 < groups) visit(key[i]);
+                } else {
+                    for (int j = prefix + lane; j < tiles; j += 32) visit(tile_key(mine[j]));
+                }
+            };
+            auto how_many = [&](uint32_t least) {
+                int count = 0;
+                each_key([&](uint32_t k) { count += k >= least; });
+                return __reduce_add_sync(0xffffffffu, count);
+            };
+            uint32_t low = 0xffffffffu, high = 0u;
+            each_key([&](uint32_t k) {
+                if (k) low = min(low, k);
+                high = max(high, k);
+            });
+            low = __reduce_min_sync(0xffffffffu, low);
+            high = __reduce_max_sync(0xffffffffu, high);
+            bool exact = false;   // exactly `keep` keys are >= low
+            if (high != 0xffffffffu) high++;
+            else if (how_many(high) >= keep) low = high;   // NaN scores
+            for (int round = 0; high - low > 1u; round++) {
+                uint32_t middle = low + (high - low) / 2;
+                if (round < 16) {
+                    const uint32_t by_value = tile_key(0.5f * key_value(low) + 0.5f * key_value(high));
+                    if (by_value > low && by_value < high) middle = by_value;
+                }
+                const int count = how_many(middle);
+                if (count >= keep) low = middle;
+                else high = middle;
+                exact = count == keep;
+                if (exact) break;
+            }
+            const uint32_t want = exact ? low - 1u : low;
+            const int greater = exact ? keep : high > low ? how_many(high) : 0;
             const int remaining = keep - greater;   // how many keys equal to `want` to take
             // Take every larger key and the first `remaining` equal keys in index order;
             // emit ascending.
             int written = 0, equal_seen = 0;
+#pragma unroll 4
             for (int base = 0; base < tiles; base += 32) {
                 const int j = base + lane;
                 bool take = false, equal = false;
@@ -232,7 +282,7 @@ score_select_kernel(const float *__restrict__ poolq, const float *__restrict__ p
                     if (j < prefix) {
                         take = true;
                     } else {
-                        const uint32_t key = sort_key(mine[j]);
+                        const uint32_t key = tile_key(mine[j]);
                         take = key > want;
                         equal = key == want;
                     }
@@ -288,47 +338,59 @@ score_select_kernel(const float *__restrict__ poolq, const float *__restrict__ p
     }
     if (!compression) return;
 
-    // ---- compression: lane owns dims 4*lane..4*lane+3 of each of its warp's query tiles ----
-    const float *pv = poolv + (size_t)head * tiles * VD;
+    // ---- compression: warp = 32 dims x 4 * QPW query tiles, thread = 4 dims x QPW query tiles ----
+    const float4 *pv = reinterpret_cast<const float4 *>(poolv + (size_t)head * tiles * VD);
+    const int dim4 = (warp & 3) * 8 + in8, q0 = (warp >> 2) * 4 * QPW + in4;
     float4 acc[QPW];
 #pragma unroll
-    for (int g = 0; g < QPW; g++) acc[g] = make_float4(0.f, 0.f, 0.f, 0.f);
-    float4 *stage4 = reinterpret_cast<float4 *>(stage);  // [CHUNK][VD/4], unpadded reuse
-    constexpr int PER_THREAD4 = CHUNK * (VD / 4) / 256;
+    for (int u = 0; u < QPW; u++) acc[u] = make_float4(0.f, 0.f, 0.f, 0.f);
+    auto add = [](float4 &a, float w, const float4 &v) {
+        a.x = fmaf(w, v.x, a.x);
+        a.y = fmaf(w, v.y, a.y);
+        a.z = fmaf(w, v.z, a.z);
+        a.w = fmaf(w, v.w, a.w);
+    };
+    float4 *stage4 = reinterpret_cast<float4 *>(stage);  // [VCHUNK][VD/4]
+    constexpr int PER_THREAD4 = VCHUNK * (VD / 4) / 256;
     float4 next4[PER_THREAD4];
     auto fetch4 = [&](int k0) {
 #pragma unroll
         for (int u = 0; u < PER_THREAD4; u++) {
             const int i = tid + u * 256, r = i / (VD / 4);
-            next4[u] = k0 + r < tiles
-                           ? __ldg(reinterpret_cast<const float4 *>(pv + (size_t)(k0 + r) * VD) + i % (VD / 4))
-                           : make_float4(0.f, 0.f, 0.f, 0.f);
+            next4[u] = k0 + r < tiles ? __ldg(pv + (size_t)(k0 + r) * (VD / 4) + i % (VD / 4))
+                                      : make_float4(0.f, 0.f, 0.f, 0.f);
         }
     };
     fetch4(0);
-    for (int k0 = 0; k0 < tiles; k0 += CHUNK) {
+    for (int k0 = 0; k0 < tiles; k0 += VCHUNK) {
         __syncthreads();
 #pragma unroll
         for (int u = 0; u < PER_THREAD4; u++) stage4[tid + u * 256] = next4[u];
         __syncthreads();
-        if (k0 + CHUNK < tiles) fetch4(k0 + CHUNK);
-        const int n = min(CHUNK, tiles - k0);
-        for (int r = 0; r < n; r++) {
-            const float4 vv = stage4[r * (VD / 4) + lane];
+        if (k0 + VCHUNK < tiles) fetch4(k0 + VCHUNK);
+        const int n = min(VCHUNK, tiles - k0), whole = n & ~3;
+#pragma unroll 2
+        for (int r = 0; r < whole; r += 4) {
+            float4 w[QPW];
 #pragma unroll
-            for (int g = 0; g < QPW; g++) {
-                const float pr = row_scores[(size_t)(warp + 8 * g) * tiles + k0 + r];
-                acc[g].x = fmaf(pr, vv.x, acc[g].x);
-                acc[g].y = fmaf(pr, vv.y, acc[g].y);
-                acc[g].z = fmaf(pr, vv.z, acc[g].z);
-                acc[g].w = fmaf(pr, vv.w, acc[g].w);
+            for (int u = 0; u < QPW; u++)
+                w[u] = *reinterpret_cast<const float4 *>(row_scores + (size_t)(q0 + 4 * u) * stride + k0 + r);
+#pragma unroll
+            for (int x = 0; x < 4; x++) {
+                const float4 v = stage4[(r + x) * (VD / 4) + dim4];
+#pragma unroll
+                for (int u = 0; u < QPW; u++) add(acc[u], x == 0 ? w[u].x : x == 1 ? w[u].y : x == 2 ? w[u].z : w[u].w, v);
             }
         }
+        for (int r = whole; r < n; r++)
+#pragma unroll
+            for (int u = 0; u < QPW; u++)
+                add(acc[u], row_scores[(size_t)(q0 + 4 * u) * stride + k0 + r], stage4[r * (VD / 4) + dim4]);
     }
 #pragma unroll
-    for (int g = 0; g < QPW; g++)
-        if (warp + 8 * g < nq)
-            reinterpret_cast<float4 *>(compression + ((size_t)head * tiles + qt0 + warp + 8 * g) * VD)[lane] = acc[g];
+    for (int u = 0; u < QPW; u++)
+        if (q0 + 4 * u < nq)
+            reinterpret_cast<float4 *>(compression + ((size_t)head * tiles + qt0 + q0 + 4 * u) * VD)[dim4] = acc[u];
 }
 
 // ---- merge ---------------------------------------------------------------------------
@@ -383,7 +445,7 @@ cudaError_t vsa_tile_pool3(const void *const src[3], void *const tiled[3], float
 }
 
 static size_t score_select_smem(int tiles, int qt) {
-    return sizeof(float) * ((size_t)qt * tiles + CHUNK * PADDED + (size_t)qt * VD);
+    return sizeof(float) * ((size_t)qt * score_stride(tiles) + KCHUNK * KPAD + (size_t)qt * QPAD);
 }
 
 template <int QPW>

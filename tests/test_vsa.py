@@ -350,6 +350,40 @@ def test_vsa_fine_extreme_logits_are_recomputed(gpu, oracle):
     assert np.abs(out - want)[:, mild].max() <= 1e-2
 
 
+@pytest.mark.parametrize("tiles,prefix,keep", [(2, 0, 1), (40, 3, 37), (65, 64, 1), (257, 1, 100), (1025, 0, 1024), (1030, 2, 77)])
+@pytest.mark.parametrize("shift", [0, 1])
+def test_vsa_select_on_pooled_values(gpu, oracle, tiles, prefix, keep, shift):
+    """The selection on its own: one video tile, all of them kept, chunk edges, more than 1024 video tiles; scores
+    that are all alike, few distinct ones, infinite and NaN ones; pooled keys that do not start on a 16-byte
+    boundary."""
+    rng = np.random.default_rng(tiles)
+    heads = 40 if tiles == 257 else 5                # enough for sixteen query tiles per CTA, or not
+    q, k = (rng.standard_normal((heads, tiles, 128)).astype(np.float32) for _ in range(2))
+    q[1] = 0.0                                       # every score zero
+    q[2, :, 1:], k[2, :, 1:] = 0.0, 0.0
+    q[2, :, 0], k[2, :, 0] = 1.0, rng.integers(-2, 3, tiles)   # five distinct scores
+    k[3, tiles // 2, 0] = np.inf                     # scores of either infinity
+    k[4, -1, 5] = np.nan
+    d = gpu.lib.h3b_tensor_data
+    tk = gpu.tensor(np.concatenate([np.zeros(shift, np.float32), k.ravel()]))
+    scores = gpu.tensor(np.zeros((heads, tiles, tiles), dtype=np.float32))
+    idx, cnt = gpu.tensor(np.full((heads, tiles, tiles), -1, np.int32)), gpu.tensor(np.zeros((heads, tiles), np.int32))
+    gpu.raw("h3b_vsa_select_raw", d(gpu.tensor(q)), d(tk) + 4 * shift, None, d(scores), d(idx), d(cnt), None, tiles,
+            prefix, keep, heads, gpu.lib.h3b_gpu_stream(gpu.gpu))
+    got_scores = gpu.read(scores, (heads, tiles, tiles), np.float32)
+    got, counts = (gpu.read_device(d(t), shape, np.int32) for t, shape in ((idx, (heads, tiles, tiles)), (cnt, (heads, tiles))))
+    bits = got_scores.view(np.uint32)
+    key = np.where(bits >> 31, ~bits, bits | np.uint32(1 << 31))      # larger score, larger key; NaN above all
+    for h in range(heads):
+        for t in range(tiles):
+            if t < prefix:
+                want = np.arange(tiles)
+            else:
+                order = np.argsort(-key[h, t, prefix:].astype(np.int64), kind="stable")[:keep]
+                want = np.concatenate([np.arange(prefix), prefix + np.sort(order)])
+            assert counts[h, t] == len(want) and np.array_equal(got[h, t, :len(want)], want), (h, t)
+
+
 @pytest.mark.parametrize("tiles,heads", [(1, 1), (2, 3), (13, 24), (64, 5), (65, 3)])
 def test_vsa_fine_walk_lengths(gpu, oracle, tiles, heads):
     """Walks of one step, of fewer and of more steps than there are score tiles and ring slots, long ones
