@@ -2,7 +2,7 @@
 // (head dim 128, h3_flash_bf16; the reference's cuda/flash_attention.cu:29-67) and the fp16 call (head
 // dim 64, h3_flash3_f16_d64, cuda/flash3_attention.cu:81-87) when the query or the output does not
 // start on a 16-byte boundary. Aligned tensors go to attn_tc5_pair.cu, which needs the boundary (TMA
-// loads, 16-byte stores) and is 5 to 10 times as fast.
+// loads, 16-byte stores) and is 4 to 6 times as fast.
 //
 // A CTA of 4 warps owns 64 query rows (16 per warp) and walks KV tiles of 64 rows staged in
 // shared memory (K row-major, V transposed so both MMA B operands are 32-bit loads).
