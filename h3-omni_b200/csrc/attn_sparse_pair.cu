@@ -382,8 +382,11 @@ attn_sparse_pair_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_
             // ------------------------------ watcher ------------------------------
             // Unit u has landed: step u - 4 may go on as far as the loads are concerned.
             if (lane == 0) {
-                int u = SP_AHEAD;
+                // (The first units, which the issuer waits for itself, are waited for here too: loads complete in
+                // any order, and the wait for a slot's second phase passes while its first is still open.)
+                int u = 0;
                 bool ok = true;
+                for (; ok && u < SP_AHEAD; u++) ok = mbar_wait_parked(bar_full(u), 0, &abort_word);
                 for (int i = 0; ok; i++) {
                     if (!mbar_wait_parked(bar_item_ready(i & 1), (i >> 1) & 1, &abort_word)) break;
                     const int n = desc[i & 1].n;
