@@ -137,10 +137,16 @@ attn_tc5_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
     const int kv_head = SPARSE ? head : head / (p.heads / p.kv_heads);
     const bool first_turn = !set_up;
     set_up = true;
-    if (!first_turn && tid == 0)
+    // (The thread that issues the loads sets the barriers up.)
+    if (!first_turn && tid == 128)
         for (int i = 0; i < 1 + 4 * ST + 2 * SB + 1; i++) mbar_inval(bar0 + 8u * i);
 
-    if (tid == 0) {
+    if (tid == 128) {
+        if (!SPARSE) {
+            tma_prefetch_desc(&map_q);
+            tma_prefetch_desc(&map_k);
+            tma_prefetch_desc(&map_v);
+        }
         mbar_init(bar_q_full(), 1);
         for (int s = 0; s < ST; s++) {
             mbar_init(bar_k_full(s), 1);
@@ -156,7 +162,20 @@ attn_tc5_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
         mbar_fence_init();
         if (first_turn) abort_word = 0;
         union_count = 0;
+        if (!SPARSE) {
+            // Requested before the CTA is complete: the latency covers the allocation of tensor memory and the barrier below.
+            mbar_arrive_expect_tx(bar_q_full(), Q_BYTES);
+            tma_load_4d(q_smem, &map_q, bar_q_full(), 0, head, q_row0, batch);
+            tma_load_4d(q_smem + Q_BYTES / 2, &map_q, bar_q_full(), 64, head, q_row0, batch);
+            mbar_arrive_expect_tx(bar_k_full(0), Cfg::TILE_BYTES);
+            tma_load_4d(k_smem, &map_k, bar_k_full(0), 0, kv_head, 0, batch);
+            tma_load_4d(k_smem + Cfg::HALF_BYTES, &map_k, bar_k_full(0), 64, kv_head, 0, batch);
+            mbar_arrive_expect_tx(bar_v_full(0), Cfg::TILE_BYTES);
+            tma_load_4d(v_smem, &map_v, bar_v_full(0), 0, kv_head, 0, batch);
+            tma_load_4d(v_smem + Cfg::HALF_BYTES, &map_v, bar_v_full(0), 64, kv_head, 0, batch);
+        }
     }
+    __syncwarp();
     if (SPARSE && tid < 128) {
         bits_a[tid] = 0;
         bits_b[tid] = 0;
@@ -230,22 +249,19 @@ attn_tc5_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
     if (warp == 4) {
         // ------------------------------ TMA producer ------------------------------
         if (lane == 0) {
-            tma_prefetch_desc(&map_q);
-            tma_prefetch_desc(&map_k);
-            tma_prefetch_desc(&map_v);
+            if (SPARSE) {
+                tma_prefetch_desc(&map_q);
+                tma_prefetch_desc(&map_k);
+                tma_prefetch_desc(&map_v);
+            }
             // (Nothing to walk: no Q either, which nobody would wait for. The barrier may be set up anew for another
             // tile, or the CTA end, while the load is still on its way.)
-            if (n_tiles > 0) {
+            if (SPARSE && n_tiles > 0) {
                 mbar_arrive_expect_tx(bar_q_full(), Q_BYTES);
-                if (SPARSE) {
-                    tma_load_4d(q_smem, &map_q, bar_q_full(), 0, q_row0, head, 0);
-                    tma_load_4d(q_smem + Q_BYTES / 2, &map_q, bar_q_full(), 64, q_row0, head, 0);
-                } else {
-                    tma_load_4d(q_smem, &map_q, bar_q_full(), 0, head, q_row0, batch);
-                    tma_load_4d(q_smem + Q_BYTES / 2, &map_q, bar_q_full(), 64, head, q_row0, batch);
-                }
+                tma_load_4d(q_smem, &map_q, bar_q_full(), 0, q_row0, head, 0);
+                tma_load_4d(q_smem + Q_BYTES / 2, &map_q, bar_q_full(), 64, q_row0, head, 0);
             }
-            for (int j = 0; j < n_tiles; j++) {
+            for (int j = SPARSE ? 0 : 1; j < n_tiles; j++) {   // (dense: tile 0 is requested above)
                 int kt, flags;
                 next_tile(j, kt, flags);
                 const int s = j % ST, use = j / ST;
@@ -452,6 +468,9 @@ attn_tc5_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
                     p.lse[((size_t)batch * p.heads + head) * p.lq + row] =
                         m_ref * p.scale + __logf(l);
             }
+            // Dense rows go through shared memory (Q's, which no MMA reads any more), so that the lanes of a warp store whole rows.
+            // (Sparse ones do not: the next turn's Q would have to be kept behind these accesses.)
+            uint4 *const stage = reinterpret_cast<uint4 *>(smem_raw + (q_smem - smem_u32(smem_raw))) + warp * 32 * 16;
             float finite = 0.0f;   // stays zero while every value is finite
 #pragma unroll
             for (int c = 0; c < HD / 32; c++) {
@@ -462,7 +481,7 @@ attn_tc5_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
 #pragma unroll
                     for (int i = 0; i < 32; i++) finite = fmaf(__uint_as_float(v[i]), 0.0f, finite);
                 }
-                if (store) {
+                if (!SPARSE || store) {
                     uint4 *d4 = reinterpret_cast<uint4 *>(dst + c * 32);
 #pragma unroll
                     for (int i = 0; i < 4; i++) {
@@ -475,8 +494,19 @@ attn_tc5_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
                                         __uint_as_float(v[i * 8 + 5]) * inv);
                         w.w = pack_bf16(__uint_as_float(v[i * 8 + 6]) * inv,
                                         __uint_as_float(v[i * 8 + 7]) * inv);
-                        d4[i] = w;
+                        if (SPARSE) d4[i] = w;
+                        else stage[lane * 16 + ((4 * c + i) ^ (lane & 7))] = w;
                     }
+                }
+            }
+            if (!SPARSE) {
+                __syncwarp();
+#pragma unroll 4
+                for (int i = 0; i < 32; i += 2) {
+                    const int local = i + (lane >> 4), row = q_row0 + warp * 32 + local;
+                    if (row >= p.lq) break;
+                    reinterpret_cast<uint4 *>(p.out + (((size_t)batch * p.lq + row) * p.heads + head) * HD)[lane & 15] =
+                        stage[local * 16 + ((lane & 15) ^ (local & 7))];
                 }
             }
             if (SPARSE && store && finite != 0.0f && listed && !alone) unsound = 1;
