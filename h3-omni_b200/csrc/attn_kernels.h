@@ -7,6 +7,25 @@ struct CUtensorMap_st;
 
 namespace h3b {
 
+// Launches a kernel that may start while the one before it in the stream still runs: its CTAs are set up as SMs become
+// free, and wait_for_previous_kernel (sm100_ptx.cuh), which every thread of it calls, keeps them off memory until then.
+// Back to back: 77 rows x 24 heads 8.19 -> 5.47 us, causal 1000 x 32 / 8 24.6 -> 23.2, fp16 4096 x 8 61.4 -> 58.6.
+template <class... Params, class... Args>
+cudaError_t launch_overlapped(void (*kernel)(Params...), dim3 grid, unsigned threads, size_t shared, cudaStream_t stream,
+                              const Args &...args) {
+    cudaLaunchConfig_t config{};
+    config.gridDim = grid;
+    config.blockDim = dim3(threads);
+    config.dynamicSmemBytes = shared;
+    config.stream = stream;
+    cudaLaunchAttribute attribute{};
+    attribute.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attribute.val.programmaticStreamSerializationAllowed = 1;
+    config.attrs = &attribute;
+    config.numAttrs = 1;
+    return cudaLaunchKernelEx(&config, kernel, args...);
+}
+
 // Address of this device's status word (0 = ok; see DeviceStatus in sm100_ptx.cuh).
 cudaError_t device_status_word(int **word);
 // Stream-ordered work memory (given back with cudaFreeAsync) from the library's pool of the current device, and

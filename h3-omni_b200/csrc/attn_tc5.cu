@@ -164,6 +164,7 @@ attn_tc5_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
         union_count = 0;
         if (!SPARSE) {
             // Requested before the CTA is complete: the latency covers the allocation of tensor memory and the barrier below.
+            wait_for_previous_kernel();
             mbar_arrive_expect_tx(bar_q_full(), Q_BYTES);
             tma_load_4d(q_smem, &map_q, bar_q_full(), 0, head, q_row0, batch);
             tma_load_4d(q_smem + Q_BYTES / 2, &map_q, bar_q_full(), 64, head, q_row0, batch);
@@ -184,10 +185,12 @@ attn_tc5_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
         tmem_alloc(smem_u32(&tmem_slot), TMEM_COLS);
         tmem_relinquish();
     }
+    if (!SPARSE) wait_for_previous_kernel();
     tc5_fence_before();
     __syncthreads();
     tc5_fence_after();
     tmem = tmem_slot;
+    if (!SPARSE && tid == 0) allow_next_kernel();
     if (SPARSE && tid == 0) unsound = 0;   // (everybody has read it, and sets it only after this thread's weights)
 
     int n_tiles;  // KV tiles this CTA walks
@@ -597,6 +600,7 @@ cudaError_t launch(const CUtensorMap &mq, const CUtensorMap &mk, const CUtensorM
         if (e != cudaSuccess) return e;
         configured_device = device;
     }
+    if (!SPARSE) return launch_overlapped(kernel, grid, TC5_THREADS, Tc5Config<BN>::SMEM_BYTES, stream, mq, mk, mv, p);
     kernel<<<grid, TC5_THREADS, Tc5Config<BN>::SMEM_BYTES, stream>>>(mq, mk, mv, p);
     return cudaGetLastError();
 }

@@ -156,9 +156,6 @@ attn_tc5_pair_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
     if (tid == 256) {
         tma_prefetch_desc(&map_q);
         tma_prefetch_desc(&kv.k[0]);
-        // A launch whose stream has already recorded a failure does nothing: when a protocol
-        // error makes every CTA run into its wait limit, the CTAs that start later leave at once.
-        const int failed = *reinterpret_cast<volatile int *>(p.status);
         mbar_init(bar_q_full, 1);
         for (int s = 0; s < ST; s++) {
             mbar_init(bar_full(s), 1);
@@ -174,6 +171,10 @@ attn_tc5_pair_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
         mbar_init(bar_pv_done, 1);
         mbar_fence_init();
         abort_word = 0;
+        wait_for_previous_kernel();
+        // A launch whose stream has already recorded a failure does nothing: when a protocol
+        // error makes every CTA run into its wait limit, the CTAs that start later leave at once.
+        const int failed = *reinterpret_cast<volatile int *>(p.status);
         mbar_arrive_expect_tx(bar_q_full, (has_b ? 2 : 1) * Cfg::Q_TILE_BYTES);
         for (int t = 0; t < (has_b ? 2 : 1); t++)
             for (int h = 0; h < Cfg::HALVES; h++)
@@ -189,10 +190,12 @@ attn_tc5_pair_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
         tmem_alloc(smem_u32(&tmem_slot), 512);
         tmem_relinquish();
     }
+    wait_for_previous_kernel();
     tc5_fence_before();
     __syncthreads();
     tc5_fence_after();
     const uint32_t tmem = tmem_slot;
+    if (tid == 0) allow_next_kernel();
 
     if (skip_launch) {
         // straight to the teardown, once what has been requested is there
@@ -582,6 +585,8 @@ attn_tc5_pair_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
 __global__ void __launch_bounds__(256)
 merge_splits_kernel(__nv_bfloat16 *__restrict__ out, float *__restrict__ lse_out, const uint4 *__restrict__ partial,
                     const float *__restrict__ lse, int splits, int lq, int heads) {
+    allow_next_kernel();
+    wait_for_previous_kernel();
     const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     const size_t total = (size_t)lq * heads * (PHD / 8);
     if (i >= total) return;
@@ -615,10 +620,9 @@ merge_splits_kernel(__nv_bfloat16 *__restrict__ out, float *__restrict__ lse_out
 cudaError_t attn_merge_splits(void *out, float *lse_out, const void *partial, const float *lse, unsigned splits,
                               unsigned lq, unsigned heads, cudaStream_t stream) {
     const size_t total = (size_t)lq * heads * (PHD / 8);
-    merge_splits_kernel<<<(unsigned)((total + 255) / 256), 256, 0, stream>>>(
-        static_cast<__nv_bfloat16 *>(out), lse_out, static_cast<const uint4 *>(partial), lse, (int)splits, (int)lq,
-        (int)heads);
-    return cudaGetLastError();
+    return launch_overlapped(merge_splits_kernel, dim3((unsigned)((total + 255) / 256)), 256, 0, stream,
+                             static_cast<__nv_bfloat16 *>(out), lse_out, static_cast<const uint4 *>(partial), lse, (int)splits,
+                             (int)lq, (int)heads);
 }
 
 namespace {
@@ -645,8 +649,7 @@ cudaError_t launch_pair(const CUtensorMap &mq, const PairKvMaps &kv, const PairP
     const unsigned pairs = ((unsigned)p.lq + 2 * PBM - 1) / (2 * PBM), heads = (unsigned)p.heads;
     if (CAUSAL && pairs > 65535u) return cudaErrorInvalidValue;
     const dim3 grid = CAUSAL ? dim3(heads, pairs, slices) : dim3(pairs, heads, slices);
-    kernel<<<grid, PAIR_THREADS, PairConfig<HD>::SMEM_BYTES, stream>>>(mq, kv, p);
-    return cudaGetLastError();
+    return launch_overlapped(kernel, grid, PAIR_THREADS, PairConfig<HD>::SMEM_BYTES, stream, mq, kv, p);
 }
 
 }  // namespace

@@ -32,6 +32,14 @@ __device__ __forceinline__ unsigned long long global_timer_ns() {
     return t;
 }
 
+// ---- launches that overlap (programmatic dependent launch) ----
+// The kernel before this one in the stream is over and what it wrote is visible. Until then a kernel that was
+// launched by launch_overlapped touches no memory that another one may use.
+__device__ __forceinline__ void wait_for_previous_kernel() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// The next kernel of the stream may be started once every CTA has got here (it waits as above). A CTA that takes tensor
+// memory calls it when it has it: the next kernel's CTAs, which hold theirs while they wait, cannot keep it from it.
+__device__ __forceinline__ void allow_next_kernel() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 // ---- mbarrier ---------------------------------------------------------------
 __device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory");

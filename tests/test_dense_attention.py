@@ -349,6 +349,35 @@ def test_causal_rows_see_nothing_of_later_values(gpu, oracle, L, key):
     assert not np.isfinite(oracle.from_bf16(got[1])[key:, :, 5]).any()
 
 
+@pytest.mark.parametrize("kind,L", [("sdpa_bf16", 77), ("sdpa_bf16", 300), ("gqa_causal_bf16", 300), ("sdpa_f16_d64", 300),
+                                    ("cross_attention_bf16", 5000)])
+def test_calls_that_overlap_see_each_other(gpu, oracle, kind, L):
+    """A kernel may be set up while the one before it runs. Calls that read what the call before wrote and write what it
+    read (query and output change places) give the bits of the same calls waited for one by one."""
+    from h3_omni_b200 import native
+    f16, H = kind == "sdpa_f16_d64", 4
+    rows, dtype = (64 if kind == "cross_attention_bf16" else L), native.F16 if f16 else native.BF16
+    rng = np.random.default_rng(L)
+    make = oracle.to_f16 if f16 else oracle.to_bf16
+    q, k, v = (make(rng.standard_normal((n, H, 64 if f16 else 128)).astype(np.float32)) for n in (rows, L, L))
+    got = []
+    for wait in (True, False):
+        a, b, tk, tv = (gpu.tensor(x, dtype) for x in (q, q, k, v))
+        for _ in range(12):
+            if kind == "cross_attention_bf16":
+                gpu.call(kind, b, 0, a, 0, tk, tv, 0, rows, L, H)
+            elif kind == "gqa_causal_bf16":
+                gpu.call(kind, b, a, tk, tv, L, H, H, 128, SCALE)
+            else:
+                gpu.call(kind, b, a, tk, tv, L, H, 64 if f16 else 128, SCALE)
+            a, b = b, a
+            if wait:
+                gpu.submit()
+        got.append(gpu.read(a, q.shape))
+    assert np.array_equal(*got)
+    assert gpu.device_status() == 0
+
+
 def test_sdpa_rejects_bad_arguments(gpu, oracle):
     """Error behaviour of the primitive layer: 0 + message, no launch."""
     q = gpu.tensor(oracle.normal_bf16((4, 2, 128), 1))
