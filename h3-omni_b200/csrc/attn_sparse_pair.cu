@@ -92,6 +92,8 @@ struct Item {
 // together hold more than half of what they could. A warp per pair, eight pairs of a head per block; both lists ascending.
 __global__ void __launch_bounds__(256)
 sparse_sums_kernel(const int *__restrict__ indices, const int *__restrict__ counts, const SparseWork work, int tiles) {
+    allow_next_kernel();
+    wait_for_previous_kernel();
     __shared__ uint32_t bits[8][SP_MAX_TILES / 32];
     __shared__ unsigned sums[2][8];   // entries and entries left, of each warp's pair
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -198,10 +200,12 @@ attn_sparse_pair_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_
         tmem_alloc(smem_u32(&tmem_slot), 512);
         tmem_relinquish();
     }
+    wait_for_previous_kernel();
     tc5_fence_before();
     __syncthreads();
     tc5_fence_after();
     const uint32_t tmem = tmem_slot;
+    if (tid == 0) allow_next_kernel();
     const int pairs = (p.tiles + 1) / 2;
 
     // Item `i`'s descriptor, for a whole warp: lane 0 polls (fewer probes of shared memory, which the
@@ -622,8 +626,8 @@ cudaError_t attn_sparse_assign(const int *indices, const int *counts, unsigned t
                                const SparseWork &work, cudaStream_t stream) {
     const cudaError_t e = cudaMemsetAsync(work.counters, 0, SparseWork::zeroed(tiles, heads), stream);
     if (e != cudaSuccess || work.assign == 0) return e;
-    sparse_sums_kernel<<<dim3(((tiles + 1) / 2 + 7) / 8, heads), 256, 0, stream>>>(indices, counts, work, (int)tiles);
-    return cudaGetLastError();
+    return launch_overlapped(sparse_sums_kernel, dim3(((tiles + 1) / 2 + 7) / 8, heads), 256, 0, stream, indices, counts, work,
+                             (int)tiles);
 }
 
 namespace {
@@ -648,8 +652,7 @@ cudaError_t launch_sparse_pair(const CUtensorMap &mk, const CUtensorMap &mv, con
     }
     const unsigned items = (unsigned)(p.tiles + 1) / 2 * (unsigned)p.heads;
     const unsigned grid = items < (unsigned)sms ? items : (unsigned)sms;   // one persistent CTA per SM
-    attn_sparse_pair_kernel<LSE><<<grid, SP_THREADS, SP_SMEM, stream>>>(mk, mv, p);
-    return cudaGetLastError();
+    return launch_overlapped(attn_sparse_pair_kernel<LSE>, dim3(grid), SP_THREADS, SP_SMEM, stream, mk, mv, p);
 }
 }  // namespace
 

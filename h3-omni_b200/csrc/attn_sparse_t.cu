@@ -197,10 +197,12 @@ attn_sparse_t_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
         tmem_alloc(smem_u32(&tmem_slot), ST_TMEM_COLS);
         tmem_relinquish();
     }
+    wait_for_previous_kernel();
     tc5_fence_before();
     __syncthreads();
     tc5_fence_after();
     const uint32_t tmem = tmem_slot;
+    if (tid == 0) allow_next_kernel();
 
     // Reads item `i`'s descriptor (waits until the scheduler has published it).
     auto fetch = [&](int i, Item &it) -> bool {
@@ -710,8 +712,7 @@ cudaError_t attn_sparse_t_launch(const CUtensorMap_st *mq, const CUtensorMap_st 
     p.scale_log2 = 0.08838834764831845f * 1.4426950408889634f;   // 1/sqrt(128), fixed by the reference kernel
     const unsigned items = tiles * heads;
     const unsigned grid = items < (unsigned)sms ? items : (unsigned)sms;   // one persistent CTA per SM
-    attn_sparse_t_kernel<<<grid, ST_THREADS, ST_SMEM, stream>>>(*mq, *mk, *mv, p);
-    return cudaGetLastError();
+    return launch_overlapped(attn_sparse_t_kernel, dim3(grid), ST_THREADS, ST_SMEM, stream, *mq, *mk, *mv, p);
 }
 
 }  // namespace h3b

@@ -97,6 +97,7 @@ attn_tc5_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
     // anything is set up. Two listed tiles of a pair go together, by the number of the even one; a tile alone has
     // rows 64-127 idle. (287 tiles x 56 heads, neighbours alike, all listed: 2.9 ms one tile at a time, 1.7 ms in pairs.)
     const bool listed = SPARSE && p.redo;
+    if (SPARSE) wait_for_previous_kernel();
     const unsigned redo_count = listed ? min(*p.redo_count, (unsigned)(p.tiles * p.heads)) : 1u;
     if (listed && blockIdx.x >= redo_count) return;
     auto in_a_pair = [&](unsigned id) -> bool {   // the other tile of its pair is listed as well
@@ -185,12 +186,12 @@ attn_tc5_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
         tmem_alloc(smem_u32(&tmem_slot), TMEM_COLS);
         tmem_relinquish();
     }
-    if (!SPARSE) wait_for_previous_kernel();
+    wait_for_previous_kernel();
     tc5_fence_before();
     __syncthreads();
     tc5_fence_after();
     tmem = tmem_slot;
-    if (!SPARSE && tid == 0) allow_next_kernel();
+    if (first_turn && tid == 0) allow_next_kernel();
     if (SPARSE && tid == 0) unsound = 0;   // (everybody has read it, and sets it only after this thread's weights)
 
     int n_tiles;  // KV tiles this CTA walks
@@ -600,9 +601,7 @@ cudaError_t launch(const CUtensorMap &mq, const CUtensorMap &mk, const CUtensorM
         if (e != cudaSuccess) return e;
         configured_device = device;
     }
-    if (!SPARSE) return launch_overlapped(kernel, grid, TC5_THREADS, Tc5Config<BN>::SMEM_BYTES, stream, mq, mk, mv, p);
-    kernel<<<grid, TC5_THREADS, Tc5Config<BN>::SMEM_BYTES, stream>>>(mq, mk, mv, p);
-    return cudaGetLastError();
+    return launch_overlapped(kernel, grid, TC5_THREADS, Tc5Config<BN>::SMEM_BYTES, stream, mq, mk, mv, p);
 }
 
 }  // namespace

@@ -155,11 +155,13 @@ out_proj_gate_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
                      : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
     }
+    wait_for_previous_kernel();
     tc5_fence_before();
     __syncthreads();
     cluster_sync();
     tc5_fence_after();
     const uint32_t tmem = tmem_slot;
+    if (tid == 0) allow_next_kernel();
     const int total = p.tiles_m * p.tiles_n, ksteps = p.inner / GK;
     const int first = blockIdx.x >> 1, stride = gridDim.x >> 1;
     // consecutive tiles share the row block (its 256 x inner slice of A stays in L2)
@@ -295,6 +297,8 @@ adaln_rows_kernel(const uint16_t *__restrict__ input, const uint16_t *__restrict
                   const uint16_t *__restrict__ modulation, const unsigned *__restrict__ row_map,
                   uint16_t *__restrict__ output, unsigned rows, unsigned width, unsigned slots, unsigned shift_slot,
                   unsigned scale_slot, float epsilon) {
+    allow_next_kernel();
+    wait_for_previous_kernel();
     const unsigned row = blockIdx.x, tid = threadIdx.x;
     if (row >= rows) return;
     __shared__ float warp_sums[4];
@@ -381,8 +385,8 @@ cudaError_t launch_proj(OutProjParams p, const void *a, const void *weight, unsi
     p.tiles_m = (p.rows + 2 * GM - 1) / (2 * GM);
     p.tiles_n = (p.hidden + GN - 1) / GN;
     const unsigned total = (unsigned)(p.tiles_m * p.tiles_n);
-    out_proj_gate_kernel<GN><<<2 * (total < sm_pairs ? total : sm_pairs), G_THREADS, ProjConfig<GN>::SMEM, stream>>>(map_a, map_b, p);
-    return cudaGetLastError();
+    return launch_overlapped(out_proj_gate_kernel<GN>, dim3(2 * (total < sm_pairs ? total : sm_pairs)), G_THREADS,
+                             ProjConfig<GN>::SMEM, stream, map_a, map_b, p);
 }
 
 }  // namespace
@@ -425,11 +429,9 @@ cudaError_t adaln_rows(void *output, const void *input, const void *norm_weight,
     if (!rows || !width || width % 4 || shift_slot >= slots || scale_slot >= slots) return cudaErrorInvalidValue;
     const unsigned chunks = (width + 511) / 512;
     auto launch = [&](auto kernel) {
-        kernel<<<rows, 128, 0, stream>>>(static_cast<const uint16_t *>(input), static_cast<const uint16_t *>(norm_weight),
-                                         static_cast<const uint16_t *>(modulation), row_map,
-                                         static_cast<uint16_t *>(output), rows, width, slots, shift_slot, scale_slot,
-                                         epsilon);
-        return cudaGetLastError();
+        return launch_overlapped(kernel, dim3(rows), 128, 0, stream, static_cast<const uint16_t *>(input),
+                                 static_cast<const uint16_t *>(norm_weight), static_cast<const uint16_t *>(modulation), row_map,
+                                 static_cast<uint16_t *>(output), rows, width, slots, shift_slot, scale_slot, epsilon);
     };
     if (chunks <= 4) return launch(adaln_rows_kernel<4>);
     if (chunks <= 8) return launch(adaln_rows_kernel<8>);

@@ -148,6 +148,8 @@ constexpr unsigned HEAD_CHUNK = 8, HEADS_IN_FLIGHT = 4;
 template <bool PEER>
 __global__ void __launch_bounds__(256, 4)
 qkv_rope_rows_kernel(const RopeArgs a) {
+    allow_next_kernel();
+    wait_for_previous_kernel();
     const unsigned lane = threadIdx.x & 31;
     const unsigned chunks = (a.heads + HEAD_CHUNK - 1) / HEAD_CHUNK;
     const size_t item = (size_t)blockIdx.x * 8 + (threadIdx.x >> 5);
@@ -211,6 +213,8 @@ qkv_rope_rows_kernel(const RopeArgs a) {
 // many instructions as the two kernels it replaces; what it saves is their memory round trip.
 __global__ void __launch_bounds__(256, 4)
 qkv_rope_tiles_kernel(const RopeArgs a) {
+    allow_next_kernel();
+    wait_for_previous_kernel();
     __shared__ float4 partial[16][3][32];   // [accumulator][tensor][lane]
     __shared__ int rows[TILE_ROWS];
     const int tile = blockIdx.x, head = blockIdx.y;
@@ -333,8 +337,7 @@ cudaError_t qkv_rope_token_major(const QkvRopeInput &in, void *q, void *k, void 
         if (reinterpret_cast<uintptr_t>(out[t]) % 8) return cudaErrorMisalignedAddress;
         a.out[t] = static_cast<uint16_t *>(out[t]);
     }
-    qkv_rope_rows_kernel<false><<<rows_grid(in), 256, 0, stream>>>(a);
-    return cudaGetLastError();
+    return launch_overlapped(qkv_rope_rows_kernel<false>, dim3(rows_grid(in)), 256, 0, stream, a);
 }
 
 cudaError_t qkv_rope_head_shards(const QkvRopeInput &in, void *const window_q[], void *const window_k[],
@@ -352,8 +355,7 @@ cudaError_t qkv_rope_head_shards(const QkvRopeInput &in, void *const window_q[],
     }
     a.rank = (unsigned)rank;
     a.ranks = (unsigned)ranks;
-    qkv_rope_rows_kernel<true><<<rows_grid(in), 256, 0, stream>>>(a);
-    return cudaGetLastError();
+    return launch_overlapped(qkv_rope_rows_kernel<true>, dim3(rows_grid(in)), 256, 0, stream, a);
 }
 
 cudaError_t qkv_rope_vsa_tiles(const QkvRopeInput &in, const int *map, const int *sizes, int tiles,
@@ -371,8 +373,7 @@ cudaError_t qkv_rope_vsa_tiles(const QkvRopeInput &in, const int *map, const int
     a.sizes = sizes;
     a.tiles = tiles;
     dim3 grid(tiles, in.heads);
-    qkv_rope_tiles_kernel<<<grid, 256, 0, stream>>>(a);
-    return cudaGetLastError();
+    return launch_overlapped(qkv_rope_tiles_kernel, grid, 256, 0, stream, a);
 }
 
 }  // namespace h3b

@@ -10,6 +10,7 @@
 #include <cstdio>
 
 #include "attn_kernels.h"
+#include "sm100_ptx.cuh"
 
 namespace h3b {
 namespace {
@@ -37,6 +38,8 @@ struct PoolArgs {
 __global__ void __launch_bounds__(256)
 tile_pool_kernel(PoolArgs a, const int *__restrict__ map, const int *__restrict__ sizes, int tiles,
                  int heads) {
+    allow_next_kernel();
+    wait_for_previous_kernel();
     __shared__ int rows[VT];
     const int tile = blockIdx.x, which = blockIdx.z;
     const int head = blockIdx.y * 8 + (threadIdx.x >> 5), dq = threadIdx.x & 31;
@@ -121,6 +124,8 @@ score_select_kernel(const float *__restrict__ poolq, const float *__restrict__ p
                     const float *__restrict__ poolv, float *__restrict__ scores_out,
                     int *__restrict__ indices, int *__restrict__ counts,
                     float *__restrict__ compression, int tiles, int prefix, int keep, float scale) {
+    allow_next_kernel();
+    wait_for_previous_kernel();
     constexpr int QT = 8 * QPW;
     extern __shared__ __align__(16) float sm[];
     const int stride = score_stride(tiles);
@@ -400,6 +405,8 @@ __global__ void __launch_bounds__(256)
 untile_merge_kernel(uint4 *__restrict__ output, const uint4 *__restrict__ tiled,
                     const uint4 *__restrict__ gate, const float *__restrict__ compression,
                     const int *__restrict__ map, int tiles, int heads) {
+    allow_next_kernel();
+    wait_for_previous_kernel();
     const size_t total = (size_t)tiles * VT * heads * (VD / 8);
     const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= total) return;
@@ -440,8 +447,7 @@ cudaError_t vsa_tile_pool3(const void *const src[3], void *const tiled[3], float
         a.pooled[i] = pooled[i];
     }
     dim3 grid(tiles, (heads + 7) / 8, count);
-    tile_pool_kernel<<<grid, 256, 0, stream>>>(a, map, sizes, tiles, heads);
-    return cudaGetLastError();
+    return launch_overlapped(tile_pool_kernel, grid, 256, 0, stream, a, map, sizes, tiles, heads);
 }
 
 static size_t score_select_smem(int tiles, int qt) {
@@ -465,9 +471,8 @@ static cudaError_t launch_score_select(const float *poolq, const float *poolk, c
         configured_device = device;
     }
     dim3 grid((tiles + QT - 1) / QT, heads);
-    score_select_kernel<QPW><<<grid, 256, score_select_smem(tiles, QT), stream>>>(
-        poolq, poolk, poolv, scores, indices, counts, compression, tiles, prefix, keep, scale);
-    return cudaGetLastError();
+    return launch_overlapped(score_select_kernel<QPW>, grid, 256, score_select_smem(tiles, QT), stream, poolq, poolk, poolv,
+                             scores, indices, counts, compression, tiles, prefix, keep, scale);
 }
 
 cudaError_t vsa_score_select_compress(const float *poolq, const float *poolk, const float *poolv,
@@ -502,10 +507,9 @@ cudaError_t vsa_untile_merge(void *output, const void *tiled, const void *gate,
     const size_t total = (size_t)tiles * VT * heads * (VD / 8);
     const size_t blocks = (total + 255) / 256;
     if (blocks > 0x7fffffffu) return cudaErrorInvalidValue;
-    untile_merge_kernel<<<(unsigned)blocks, 256, 0, stream>>>(
-        static_cast<uint4 *>(output), static_cast<const uint4 *>(tiled),
-        static_cast<const uint4 *>(gate), compression, map, tiles, heads);
-    return cudaGetLastError();
+    return launch_overlapped(untile_merge_kernel, dim3((unsigned)blocks), 256, 0, stream, static_cast<uint4 *>(output),
+                             static_cast<const uint4 *>(tiled), static_cast<const uint4 *>(gate), compression, map, tiles,
+                             heads);
 }
 
 }  // namespace h3b
