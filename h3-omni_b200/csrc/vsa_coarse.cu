@@ -86,8 +86,8 @@ tile_pool_kernel(PoolArgs a, const int *__restrict__ map, const int *__restrict_
 }
 
 // ---- scores + top-k selection + compression -----------------------------------------
-constexpr int KCHUNK = 128, KHALF = 64;   // pooled K staged per step: 128 rows x 64 dims
-constexpr int KPAD = KHALF + 4;           // rows 4 banks apart: 8 rows x 16 bytes hit 32 distinct banks
+constexpr int KCHUNK = 256, KPART = 32;   // pooled K staged per step: 256 rows x 32 dims
+constexpr int KPAD = KPART + 4;           // rows 4 banks apart: 8 rows x 16 bytes hit 32 distinct banks
 constexpr int QPAD = VD + 4;
 constexpr int VCHUNK = 64;                // pooled V rows staged per step
 static_assert(VCHUNK * VD <= KCHUNK * KPAD, "V stage fits the K stage");
@@ -112,12 +112,13 @@ __device__ __forceinline__ float key_value(uint32_t k) {
 //   all prefix tiles plus the `keep` best video tiles (ties: lower index first), ascending.
 //   Compression (cuda/vsa.cuh:80-166,291-294): softmax over the whole row in the ATen lane
 //   order, then sum_k p[k] * poolv[k][:] as one fmaf chain over k ascending.
-// Both products are bound by shared-memory wavefronts unless a read feeds several FMAs: a warp covers 8 rows
-// (or 8 x 4 dims) by 4 query tiles, so that a vector read is one wavefront, broadcast to the other lanes, and
-// a thread takes 4 keys x QPW query tiles of the scores (4 + QPW wavefronts per 16 * QPW FMAs) and 4 dims x
-// QPW query tiles of the compression (4 + QPW per 4 keys and 16 * QPW FMAs).
-// 905 tiles x 24 heads: 754 us with a key row (or four dims) per lane and a bit-by-bit search, 704 with this tiling,
-// 660 with the interval search below (287 tiles x 56 heads: 231 -> 198 for the search).
+// Both products are bound by shared-memory reads unless a read feeds several FMAs: a warp covers 8 rows
+// (or 8 x 4 dims) by 4 query tiles, so that the lanes of a vector read share addresses, and a thread takes 4 keys x 2 QPW
+// query tiles of the scores (4 + 2 QPW reads per 32 * QPW FMAs) and 4 dims x QPW query tiles of the compression (4 + QPW
+// per 4 keys and 16 * QPW FMAs).
+// 905 tiles x 24 heads: 754 us with a key row (or four dims) per lane and a bit-by-bit search, 704 with four keys x QPW
+// query tiles per thread, 660 with the interval search below. With 2 QPW query tiles per thread (256 keys x 32 dims
+// staged instead of 128 x 64) whole calls of 450 tiles x 14 heads take 1606 us instead of 1633, 50 x 3 70.5 instead of 72.3.
 template <int QPW>
 __global__ void __launch_bounds__(256, 2)
 score_select_kernel(const float *__restrict__ poolq, const float *__restrict__ poolk,
@@ -142,17 +143,17 @@ score_select_kernel(const float *__restrict__ poolq, const float *__restrict__ p
         const int qi = i / VD, d = i % VD;
         qrows[qi * QPAD + d] = qi < nq ? poolq[((size_t)head * tiles + qt0 + qi) * VD + d] : 0.0f;
     }
-    // ---- scores: warp = 32 keys (of 128) x 4 * QPW query tiles ----
+    // ---- scores: warp = 32 keys (of 256) x all query tiles ----
     {
         const float *pk = poolk + (size_t)head * tiles * VD;
         const bool wide = reinterpret_cast<uintptr_t>(poolk) % 16 == 0;   // a caller's own array need not be
-        constexpr int PER_THREAD = KCHUNK * KHALF / 4 / 256;
+        constexpr int PER_THREAD = KCHUNK * KPART / 4 / 256, NQ = 2 * QPW;
         float4 next[PER_THREAD];   // this thread's part of the stage being fetched
-        auto fetch = [&](int k0, int half) {
+        auto fetch = [&](int k0, int part) {
 #pragma unroll
             for (int u = 0; u < PER_THREAD; u++) {
-                const int i = tid + u * 256, r = i / (KHALF / 4), c = i % (KHALF / 4);
-                const float *at = pk + (size_t)(k0 + r) * VD + half * KHALF + c * 4;
+                const int i = tid + u * 256, r = i / (KPART / 4), c = i % (KPART / 4);
+                const float *at = pk + (size_t)(k0 + r) * VD + part * KPART + c * 4;
                 next[u] = make_float4(0.f, 0.f, 0.f, 0.f);
                 if (k0 + r < tiles)
                     next[u] = wide ? __ldg(reinterpret_cast<const float4 *>(at))
@@ -160,36 +161,38 @@ score_select_kernel(const float *__restrict__ poolq, const float *__restrict__ p
             }
         };
         fetch(0, 0);
-        const int key0 = (warp >> 1) * 32 + in8, q0 = (warp & 1) * 4 * QPW + in4;
+        const int key0 = warp * 32 + in8, q0 = in4;
         for (int k0 = 0; k0 < tiles; k0 += KCHUNK) {
-            float dot[4][QPW];
+            const bool busy = k0 + warp * 32 < tiles;   // the last chunk may have no keys for a warp
+            float dot[4][NQ];
 #pragma unroll
             for (int i = 0; i < 4; i++)
 #pragma unroll
-                for (int u = 0; u < QPW; u++) dot[i][u] = 0.0f;
+                for (int u = 0; u < NQ; u++) dot[i][u] = 0.0f;
 #pragma unroll 1
-            for (int half = 0; half < 2; half++) {
+            for (int part = 0; part < VD / KPART; part++) {
                 __syncthreads();   // the stage is used up
 #pragma unroll
                 for (int u = 0; u < PER_THREAD; u++) {
                     const int i = tid + u * 256;
-                    *reinterpret_cast<float4 *>(stage + (i / (KHALF / 4)) * KPAD + (i % (KHALF / 4)) * 4) = next[u];
+                    *reinterpret_cast<float4 *>(stage + (i / (KPART / 4)) * KPAD + (i % (KPART / 4)) * 4) = next[u];
                 }
                 __syncthreads();
-                if (half == 0) fetch(k0, 1);
+                if (part + 1 < VD / KPART) fetch(k0, part + 1);
                 else if (k0 + KCHUNK < tiles) fetch(k0 + KCHUNK, 0);
-#pragma unroll 4
-                for (int d = 0; d < KHALF; d += 4) {
-                    float4 kv[4], qv[QPW];
+                if (!busy) continue;
+#pragma unroll 2
+                for (int d = 0; d < KPART; d += 4) {
+                    float4 kv[4], qv[NQ];
 #pragma unroll
                     for (int i = 0; i < 4; i++) kv[i] = *reinterpret_cast<const float4 *>(stage + (key0 + 8 * i) * KPAD + d);
 #pragma unroll
-                    for (int u = 0; u < QPW; u++)
-                        qv[u] = *reinterpret_cast<const float4 *>(qrows + (q0 + 4 * u) * QPAD + half * KHALF + d);
+                    for (int u = 0; u < NQ; u++)
+                        qv[u] = *reinterpret_cast<const float4 *>(qrows + (q0 + 4 * u) * QPAD + part * KPART + d);
 #pragma unroll
                     for (int i = 0; i < 4; i++)
 #pragma unroll
-                        for (int u = 0; u < QPW; u++) {
+                        for (int u = 0; u < NQ; u++) {
                             dot[i][u] = fmaf(qv[u].x, kv[i].x, dot[i][u]);
                             dot[i][u] = fmaf(qv[u].y, kv[i].y, dot[i][u]);
                             dot[i][u] = fmaf(qv[u].z, kv[i].z, dot[i][u]);
@@ -200,7 +203,7 @@ score_select_kernel(const float *__restrict__ poolq, const float *__restrict__ p
 #pragma unroll
             for (int i = 0; i < 4; i++)
 #pragma unroll
-                for (int u = 0; u < QPW; u++)
+                for (int u = 0; u < NQ; u++)
                     if (k0 + key0 + 8 * i < tiles && q0 + 4 * u < nq)
                         row_scores[(size_t)(q0 + 4 * u) * stride + k0 + key0 + 8 * i] = scale * dot[i][u];
         }
@@ -481,7 +484,7 @@ cudaError_t vsa_score_select_compress(const float *poolq, const float *poolk, co
                                       int heads, float scale, cudaStream_t stream) {
     if (tiles < 1 || tiles > 4096 || keep < 1 || prefix < 0 || prefix > tiles)
         return cudaErrorInvalidValue;
-    // 16 query tiles per CTA up to 1400 tiles (two such CTAs share an SM up to about 1130 tiles,
+    // 16 query tiles per CTA up to 1400 tiles (two such CTAs share an SM up to about 1090 tiles,
     // one beyond), 8 per CTA beyond that: the score rows of a CTA must fit its shared memory.
     // A CTA's time is its own chain of chunks (products bound by shared-memory wavefronts, a dozen counts per query
     // tile for the threshold), so a call takes about one CTA's time as long as every CTA is resident: with few
