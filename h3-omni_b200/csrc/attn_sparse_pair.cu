@@ -91,9 +91,9 @@ struct Item {
 // Sums for the choice between the kernels (sparse_choice.cuh), and the list of long pairs: those whose lists
 // together hold more than half of what they could. A warp per pair, eight pairs of a head per block; both lists ascending.
 __global__ void __launch_bounds__(256)
-sparse_sums_kernel(const int *__restrict__ indices, const int *__restrict__ counts, const SparseWork work, int tiles) {
-    allow_next_kernel();
+sparse_sums_kernel(const int *indices, const int *counts, const SparseWork work, int tiles) {
     wait_for_previous_kernel();
+    allow_next_kernel();
     __shared__ uint32_t bits[8][SP_MAX_TILES / 32];
     __shared__ unsigned sums[2][8];   // entries and entries left, of each warp's pair
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -458,7 +458,7 @@ attn_sparse_pair_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_
                 uint32_t v[32];
 #pragma unroll
                 for (int x = 0; x < 8; x++) {
-                    const uint4 w = real ? __ldg(src + c * 8 + x) : make_uint4(0u, 0u, 0u, 0u);
+                    const uint4 w = real ? src[c * 8 + x] : make_uint4(0u, 0u, 0u, 0u);
                     v[4 * x] = w.x;
                     v[4 * x + 1] = w.y;
                     v[4 * x + 2] = w.z;

@@ -583,10 +583,10 @@ attn_tc5_pair_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
 // Combines the slices of a split-KV call: out[r][h][:] = sum_s w_s O_s[r][h][:] / sum_s w_s with
 // w_s = exp(lse_s - max_s lse_s). One thread per (row, head, eight dims).
 __global__ void __launch_bounds__(256)
-merge_splits_kernel(__nv_bfloat16 *__restrict__ out, float *__restrict__ lse_out, const uint4 *__restrict__ partial,
-                    const float *__restrict__ lse, int splits, int lq, int heads) {
-    allow_next_kernel();
+merge_splits_kernel(__nv_bfloat16 *out, float *lse_out, const uint4 *partial, const float *lse, int splits, int lq,
+                    int heads) {
     wait_for_previous_kernel();
+    allow_next_kernel();
     const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     const size_t total = (size_t)lq * heads * (PHD / 8);
     if (i >= total) return;

@@ -293,12 +293,11 @@ out_proj_gate_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
 // tree, warp sums paired (0+2, 1+3), then (0+1).
 template <int CHUNKS>
 __global__ void __launch_bounds__(128)
-adaln_rows_kernel(const uint16_t *__restrict__ input, const uint16_t *__restrict__ weight,
-                  const uint16_t *__restrict__ modulation, const unsigned *__restrict__ row_map,
-                  uint16_t *__restrict__ output, unsigned rows, unsigned width, unsigned slots, unsigned shift_slot,
+adaln_rows_kernel(const uint16_t *input, const uint16_t *weight, const uint16_t *modulation, const unsigned *row_map,
+                  uint16_t *output, unsigned rows, unsigned width, unsigned slots, unsigned shift_slot,
                   unsigned scale_slot, float epsilon) {
-    allow_next_kernel();
     wait_for_previous_kernel();
+    allow_next_kernel();
     const unsigned row = blockIdx.x, tid = threadIdx.x;
     if (row >= rows) return;
     __shared__ float warp_sums[4];

@@ -59,8 +59,8 @@ struct LaneSetup {
 };
 
 __device__ __forceinline__ void lane_weights(const RopeArgs &a, unsigned lane, LaneSetup &u) {
-    unpack4(__ldg(reinterpret_cast<const uint2 *>(a.q_weight) + lane), u.qw);
-    unpack4(__ldg(reinterpret_cast<const uint2 *>(a.k_weight) + lane), u.kw);
+    unpack4(reinterpret_cast<const uint2 *>(a.q_weight)[lane], u.qw);
+    unpack4(reinterpret_cast<const uint2 *>(a.k_weight)[lane], u.kw);
     const unsigned quarter = a.rope_half / 4;
     u.role = lane < quarter ? 0 : lane < 2 * quarter ? 1 : 2;
     u.partner = u.role == 0 ? lane + quarter : u.role == 1 ? lane - quarter : lane;
@@ -72,8 +72,8 @@ __device__ __forceinline__ void load_angles(const RopeArgs &a, unsigned lane, co
     c = s = make_uint2(0u, 0u);
     if (u.role == 2) return;
     const size_t angle = row * a.rope_half + (u.role == 0 ? lane * 4 : lane * 4 - a.rope_half);
-    c = __ldg(reinterpret_cast<const uint2 *>(a.rope_cos + angle));
-    s = __ldg(reinterpret_cast<const uint2 *>(a.rope_sin + angle));
+    c = *reinterpret_cast<const uint2 *>(a.rope_cos + angle);
+    s = *reinterpret_cast<const uint2 *>(a.rope_sin + angle);
 }
 __device__ __forceinline__ void set_angles(LaneSetup &u, uint2 c, uint2 s) {
     u.c = c;
@@ -148,8 +148,8 @@ constexpr unsigned HEAD_CHUNK = 8, HEADS_IN_FLIGHT = 4;
 template <bool PEER>
 __global__ void __launch_bounds__(256, 4)
 qkv_rope_rows_kernel(const RopeArgs a) {
-    allow_next_kernel();
     wait_for_previous_kernel();
+    allow_next_kernel();
     const unsigned lane = threadIdx.x & 31;
     const unsigned chunks = (a.heads + HEAD_CHUNK - 1) / HEAD_CHUNK;
     const size_t item = (size_t)blockIdx.x * 8 + (threadIdx.x >> 5);
@@ -213,8 +213,8 @@ qkv_rope_rows_kernel(const RopeArgs a) {
 // many instructions as the two kernels it replaces; what it saves is their memory round trip.
 __global__ void __launch_bounds__(256, 4)
 qkv_rope_tiles_kernel(const RopeArgs a) {
-    allow_next_kernel();
     wait_for_previous_kernel();
+    allow_next_kernel();
     __shared__ float4 partial[16][3][32];   // [accumulator][tensor][lane]
     __shared__ int rows[TILE_ROWS];
     const int tile = blockIdx.x, head = blockIdx.y;

@@ -34,9 +34,13 @@ __device__ __forceinline__ unsigned long long global_timer_ns() {
 
 // ---- launches that overlap (programmatic dependent launch) ----
 // The kernel before this one in the stream is over and what it wrote is visible. Until then a kernel that was
-// launched by launch_overlapped touches no memory that another one may use.
+// launched by launch_overlapped touches no memory that another one may use. What the wait makes visible it makes
+// visible to ordinary loads: such a kernel has begun before its inputs are complete, so it may not read them through the
+// read-only path (__ldg, or const __restrict__ parameters, for which the compiler takes that path), which is specified
+// for data that does not change while the kernel runs.
 __device__ __forceinline__ void wait_for_previous_kernel() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-// The next kernel of the stream may be started once every CTA has got here (it waits as above). A CTA that takes tensor
+// The next kernel of the stream may be started once every CTA has got here (it waits as above). After the wait: no
+// kernel then starts before the last but one is over. A CTA that takes tensor
 // memory calls it when it has it: the next kernel's CTAs, which hold theirs while they wait, cannot keep it from it.
 __device__ __forceinline__ void allow_next_kernel() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 

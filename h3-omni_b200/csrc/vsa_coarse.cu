@@ -25,8 +25,12 @@ __device__ __forceinline__ float bf16_round(float x) { return bf16_bits_to_f32(f
 
 // ---- pooling ---------------------------------------------------------------------
 // One CTA = one tile x 8 heads x one of {Q, K, V}; thread = (head, four dims = 8 bytes), so
-// every token row contributes one contiguous 2 KB read per CTA and each thread keeps 64
-// independent 8-byte loads in flight. The per-dimension summation order is the reference's
+// every token row contributes one contiguous 2 KB read per CTA. Bound by HBM: a thread requests 32 rows before it
+// stores the first of them (a load does not move up across a store that may be to the same place). The loop over
+// the two halves stays rolled, or all 64 row numbers are held at once and one CTA fits an SM instead of two.
+// 287 tiles x 56 heads: 266 us with all loads through the read-only path, 243 so; 905 x 24 362 -> 328; 144 x 14
+// 37.2 -> 33.9; 50 x 7 6.9 -> 7.6. (One lane at a time, three CTAs per SM: 247, 334, 34.1 and 9.3.)
+// The per-dimension summation order is the reference's
 // (cuda/vsa.cuh:22-42): 4 lanes x 4 slot accumulators, element i = lane + 4*slot + 16*round,
 // ((a0+a1)+a2)+a3 per lane, (l0+l2)+(l1+l3), then / size.
 struct PoolArgs {
@@ -35,11 +39,11 @@ struct PoolArgs {
     float *pooled[3];
 };
 
-__global__ void __launch_bounds__(256)
-tile_pool_kernel(PoolArgs a, const int *__restrict__ map, const int *__restrict__ sizes, int tiles,
-                 int heads) {
-    allow_next_kernel();
+template <bool TILED>
+__global__ void __launch_bounds__(256, 2)
+tile_pool_kernel(PoolArgs a, const int *map, const int *sizes, int tiles, int heads) {
     wait_for_previous_kernel();
+    allow_next_kernel();
     __shared__ int rows[VT];
     const int tile = blockIdx.x, which = blockIdx.z;
     const int head = blockIdx.y * 8 + (threadIdx.x >> 5), dq = threadIdx.x & 31;
@@ -49,39 +53,49 @@ tile_pool_kernel(PoolArgs a, const int *__restrict__ map, const int *__restrict_
     const uint2 *src = which == 0 ? a.src[0] : which == 1 ? a.src[1] : a.src[2];
     uint2 *tiled = which == 0 ? a.tiled[0] : which == 1 ? a.tiled[1] : a.tiled[2];
     float *pooled = which == 0 ? a.pooled[0] : which == 1 ? a.pooled[1] : a.pooled[2];
-    float lane_sum[4][4];   // [lane][dim]
+    float even[4], sum[4];   // lanes 0 and 2; the two lanes of this turn
+#pragma unroll 1
+    for (int first = 0; first < 2; first++) {
+        uint2 held[2][16];   // [lane / 2][slot + 4 * round]
 #pragma unroll
-    for (int lane = 0; lane < 4; lane++) {
-        float acc[4][4];    // [slot][dim]
-#pragma unroll
-        for (int slot = 0; slot < 4; slot++)
-#pragma unroll
-            for (int d = 0; d < 4; d++) acc[slot][d] = 0.0f;
-#pragma unroll
-        for (int round = 0; round < 4; round++) {
-#pragma unroll
-            for (int slot = 0; slot < 4; slot++) {
-                const int i = lane + slot * 4 + round * 16;
-                const int row = rows[i];
-                uint2 x = make_uint2(0u, 0u);
-                if (row >= 0) x = __ldg(src + ((size_t)row * heads + head) * (VD / 4) + dq);
-                if (tiled) tiled[((size_t)head * tiles * VT + tile * VT + i) * (VD / 4) + dq] = x;
-                acc[slot][0] += bf16_bits_to_f32(x.x & 0xffffu);
-                acc[slot][1] += bf16_bits_to_f32(x.x >> 16);
-                acc[slot][2] += bf16_bits_to_f32(x.y & 0xffffu);
-                acc[slot][3] += bf16_bits_to_f32(x.y >> 16);
-            }
+        for (int n = 0; n < 32; n++) {
+            const int row = rows[first + 2 * (n / 16) + 4 * (n % 16)];
+            held[n / 16][n % 16] = make_uint2(0u, 0u);
+            if (row >= 0) held[n / 16][n % 16] = src[((size_t)row * heads + head) * (VD / 4) + dq];
         }
 #pragma unroll
-        for (int d = 0; d < 4; d++)
-            lane_sum[lane][d] = ((acc[0][d] + acc[1][d]) + acc[2][d]) + acc[3][d];
+        for (int which_lane = 0; which_lane < 2; which_lane++) {
+            const int lane = first + 2 * which_lane;
+            float acc[4][4];   // [slot][dim]
+#pragma unroll
+            for (int slot = 0; slot < 4; slot++)
+#pragma unroll
+                for (int d = 0; d < 4; d++) acc[slot][d] = 0.0f;
+#pragma unroll
+            for (int n = 0; n < 16; n++) {
+                const uint2 x = held[which_lane][n];
+                if (TILED) tiled[((size_t)head * tiles * VT + tile * VT + lane + 4 * n) * (VD / 4) + dq] = x;
+                acc[n % 4][0] += bf16_bits_to_f32(x.x & 0xffffu);
+                acc[n % 4][1] += bf16_bits_to_f32(x.x >> 16);
+                acc[n % 4][2] += bf16_bits_to_f32(x.y & 0xffffu);
+                acc[n % 4][3] += bf16_bits_to_f32(x.y >> 16);
+            }
+#pragma unroll
+            for (int d = 0; d < 4; d++) {
+                const float own = ((acc[0][d] + acc[1][d]) + acc[2][d]) + acc[3][d];
+                sum[d] = which_lane ? sum[d] + own : own;
+            }
+        }
+        if (first == 0)
+#pragma unroll
+            for (int d = 0; d < 4; d++) even[d] = sum[d];
     }
     const float size = (float)sizes[tile];
     float4 mean;
-    mean.x = ((lane_sum[0][0] + lane_sum[2][0]) + (lane_sum[1][0] + lane_sum[3][0])) / size;
-    mean.y = ((lane_sum[0][1] + lane_sum[2][1]) + (lane_sum[1][1] + lane_sum[3][1])) / size;
-    mean.z = ((lane_sum[0][2] + lane_sum[2][2]) + (lane_sum[1][2] + lane_sum[3][2])) / size;
-    mean.w = ((lane_sum[0][3] + lane_sum[2][3]) + (lane_sum[1][3] + lane_sum[3][3])) / size;
+    mean.x = (even[0] + sum[0]) / size;
+    mean.y = (even[1] + sum[1]) / size;
+    mean.z = (even[2] + sum[2]) / size;
+    mean.w = (even[3] + sum[3]) / size;
     reinterpret_cast<float4 *>(pooled)[((size_t)head * tiles + tile) * (VD / 4) + dq] = mean;
 }
 
@@ -121,12 +135,10 @@ __device__ __forceinline__ float key_value(uint32_t k) {
 // staged instead of 128 x 64) whole calls of 450 tiles x 14 heads take 1606 us instead of 1633, 50 x 3 70.5 instead of 72.3.
 template <int QPW>
 __global__ void __launch_bounds__(256, 2)
-score_select_kernel(const float *__restrict__ poolq, const float *__restrict__ poolk,
-                    const float *__restrict__ poolv, float *__restrict__ scores_out,
-                    int *__restrict__ indices, int *__restrict__ counts,
-                    float *__restrict__ compression, int tiles, int prefix, int keep, float scale) {
-    allow_next_kernel();
+score_select_kernel(const float *poolq, const float *poolk, const float *poolv, float *scores_out, int *indices,
+                    int *counts, float *compression, int tiles, int prefix, int keep, float scale) {
     wait_for_previous_kernel();
+    allow_next_kernel();
     constexpr int QT = 8 * QPW;
     extern __shared__ __align__(16) float sm[];
     const int stride = score_stride(tiles);
@@ -156,8 +168,7 @@ score_select_kernel(const float *__restrict__ poolq, const float *__restrict__ p
                 const float *at = pk + (size_t)(k0 + r) * VD + part * KPART + c * 4;
                 next[u] = make_float4(0.f, 0.f, 0.f, 0.f);
                 if (k0 + r < tiles)
-                    next[u] = wide ? __ldg(reinterpret_cast<const float4 *>(at))
-                                   : make_float4(__ldg(at), __ldg(at + 1), __ldg(at + 2), __ldg(at + 3));
+                    next[u] = wide ? *reinterpret_cast<const float4 *>(at) : make_float4(at[0], at[1], at[2], at[3]);
             }
         };
         fetch(0, 0);
@@ -365,8 +376,7 @@ score_select_kernel(const float *__restrict__ poolq, const float *__restrict__ p
 #pragma unroll
         for (int u = 0; u < PER_THREAD4; u++) {
             const int i = tid + u * 256, r = i / (VD / 4);
-            next4[u] = k0 + r < tiles ? __ldg(pv + (size_t)(k0 + r) * (VD / 4) + i % (VD / 4))
-                                      : make_float4(0.f, 0.f, 0.f, 0.f);
+            next4[u] = k0 + r < tiles ? pv[(size_t)(k0 + r) * (VD / 4) + i % (VD / 4)] : make_float4(0.f, 0.f, 0.f, 0.f);
         }
     };
     fetch4(0);
@@ -405,11 +415,10 @@ score_select_kernel(const float *__restrict__ poolq, const float *__restrict__ p
 // out[row][h][:] = bf16(fmaf(bf16_round(compression[h][tile][:]), gate[row][h][:], sparse))
 // for every non-padded tiled row (cuda/vsa.cuh:168-181); one 16-byte vector per thread.
 __global__ void __launch_bounds__(256)
-untile_merge_kernel(uint4 *__restrict__ output, const uint4 *__restrict__ tiled,
-                    const uint4 *__restrict__ gate, const float *__restrict__ compression,
-                    const int *__restrict__ map, int tiles, int heads) {
-    allow_next_kernel();
+untile_merge_kernel(uint4 *output, const uint4 *tiled, const uint4 *gate, const float *compression, const int *map,
+                    int tiles, int heads) {
     wait_for_previous_kernel();
+    allow_next_kernel();
     const size_t total = (size_t)tiles * VT * heads * (VD / 8);
     const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= total) return;
@@ -450,7 +459,8 @@ cudaError_t vsa_tile_pool3(const void *const src[3], void *const tiled[3], float
         a.pooled[i] = pooled[i];
     }
     dim3 grid(tiles, (heads + 7) / 8, count);
-    return launch_overlapped(tile_pool_kernel, grid, 256, 0, stream, a, map, sizes, tiles, heads);
+    return launch_overlapped(a.tiled[0] ? tile_pool_kernel<true> : tile_pool_kernel<false>, grid, 256, 0, stream, a, map, sizes,
+                             tiles, heads);
 }
 
 static size_t score_select_smem(int tiles, int qt) {
