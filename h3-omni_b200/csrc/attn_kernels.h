@@ -25,7 +25,9 @@ cudaError_t launch_overlapped(void (*kernel)(Params...), dim3 grid, unsigned thr
     attribute.val.programmaticStreamSerializationAllowed = 1;
     config.attrs = &attribute;
     config.numAttrs = 1;
-    return cudaLaunchKernelEx(&config, kernel, args...);
+    const cudaError_t e = cudaLaunchKernelEx(&config, kernel, args...);
+    if (e != cudaSuccess) cudaGetLastError();   // the caller has the code; the next launch's check must not find it
+    return e;
 }
 
 // Address of this device's status word (0 = ok; see DeviceStatus in sm100_ptx.cuh).

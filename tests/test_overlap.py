@@ -88,3 +88,24 @@ def test_static_topk_in_a_row_with_changing_inputs(gpu, oracle, busy, heads, sha
         assert gpu.device_status() == 0
     finally:
         gpu.lib.h3_gpu_vsa_free(handle)
+
+
+@pytest.mark.gpu
+def test_a_refused_launch_leaves_no_error_behind(gpu, oracle):
+    """A grid of more heads than the launch takes is refused by the runtime. The code comes back from that call, and the
+    next one, a kernel launched and checked in the ordinary way (an output off 16-byte boundaries), succeeds."""
+    heads, L = 65536, 20
+    data, stream = gpu.lib.h3b_tensor_data, gpu.lib.h3b_gpu_stream(gpu.gpu)
+    pooled = gpu.tensor(np.zeros((heads, 1, 128), dtype=np.float32))
+    lists = [gpu.tensor(np.full(heads, -7, dtype=np.int32)) for _ in range(2)]
+    q, k, v = (gpu.tensor(oracle.normal_bf16((L, 1, 128), 71 + i)) for i in range(3))
+    want, out = gpu.tensor(np.zeros((L, 128), dtype=np.uint16)), gpu.tensor(np.zeros((L + 1, 128), dtype=np.uint16))
+    assert gpu.lib.h3b_vsa_select_raw(data(pooled), data(pooled), None, None, data(lists[0]), data(lists[1]), None, 1, 0, 1,
+                                      heads, stream) != 0
+    gpu.raw("h3_flash_bf16", data(out) + 4, data(q), data(k), data(v), None, 1, L, 1, 1, 0.0883883476, True, stream)
+    gpu.raw("h3_flash_bf16", data(want), data(q), data(k), data(v), None, 1, L, 1, 1, 0.0883883476, True, stream)
+    got = gpu.read(out, ((L + 1) * 128,))[2:2 + L * 128]
+    # Values below 4: either result is within half a bf16 step (2^-7) and its weights' rounding (2^-9 of 4) of the exact one.
+    got, want = oracle.from_bf16(got), oracle.from_bf16(gpu.read(want, (L * 128,)))
+    assert np.abs(want).max() < 4 and np.abs(got - want).max() <= 2.0 ** -5
+    assert all(np.array_equal(gpu.read(t, (heads,), np.int32), np.full(heads, -7, dtype=np.int32)) for t in lists)
