@@ -101,12 +101,22 @@ tile_pool_kernel(PoolArgs a, const int *map, const int *sizes, int tiles, int he
 
 // ---- scores + top-k selection + compression -----------------------------------------
 constexpr int KCHUNK = 256, KPART = 32;   // pooled K staged per step: 256 rows x 32 dims
-constexpr int KPAD = KPART + 4;           // rows 4 banks apart: 8 rows x 16 bytes hit 32 distinct banks
-constexpr int QPAD = VD + 4;
+constexpr int QPAD = VD + 4;              // rows 4 banks apart
 constexpr int VCHUNK = 64;                // pooled V rows staged per step
-static_assert(VCHUNK * VD <= KCHUNK * KPAD, "V stage fits the K stage");
+static_assert(VCHUNK * VD <= KCHUNK * KPART, "V stage fits the K stage");
+// Where dims d .. d + 3 of row r are staged: the eight 16-byte pieces of a row change places with the row's number, so
+// that 8 rows x 16 bytes hit 32 distinct banks without padding.
+__device__ __forceinline__ int staged(int r, int d) { return r * KPART + (d ^ (r & 7) * 4); }
 // Floats between two score rows: float4-aligned and 4 banks apart like the rows above.
 __host__ __device__ constexpr int score_stride(int tiles) { return (tiles + 31) / 32 * 32 + 4; }
+constexpr size_t score_select_smem(int tiles, int qt) {
+    return sizeof(float) * ((size_t)qt * score_stride(tiles) + KCHUNK * KPART + (size_t)qt * QPAD);
+}
+// Two CTAs of 16 query tiles share an SM's 228 KB (1 KB of which each CTA's launch takes) up to 1152 tiles, two of 8 up to 2432.
+// Where one has it to itself a call takes a third longer: 24 heads of 1120 tiles 1235 us with one, 905 with two; of 1152 940
+// and of 1160 1290; 8 heads of 2390 tiles 2774 and 2031.
+static_assert(2 * (score_select_smem(1152, 16) + 1024) <= 228 * 1024 && 2 * (score_select_smem(2432, 8) + 1024) <= 228 * 1024,
+              "two CTAs per SM");
 
 // Order-preserving key of a float, the one cub's radix sort uses: larger float -> larger key.
 __device__ __forceinline__ uint32_t sort_key(float f) {
@@ -131,8 +141,9 @@ __device__ __forceinline__ float key_value(uint32_t k) {
 // query tiles of the scores (4 + 2 QPW reads per 32 * QPW FMAs) and 4 dims x QPW query tiles of the compression (4 + QPW
 // per 4 keys and 16 * QPW FMAs).
 // 905 tiles x 24 heads: 754 us with a key row (or four dims) per lane and a bit-by-bit search, 704 with four keys x QPW
-// query tiles per thread, 660 with the interval search below. With 2 QPW query tiles per thread (256 keys x 32 dims
-// staged instead of 128 x 64) whole calls of 450 tiles x 14 heads take 1606 us instead of 1633, 50 x 3 70.5 instead of 72.3.
+// query tiles per thread, 644 with the interval search below, 582 with 2 QPW query tiles per thread (256 keys x 32 dims
+// staged instead of 128 x 64), 560 with ordinary loads and the dims of a part unrolled. 450 x 14: 172, 146, 142 us in the last three steps,
+// 287 x 56 189, 177, 170, 50 x 3 12.1, 11.7, 11.4.
 template <int QPW>
 __global__ void __launch_bounds__(256, 2)
 score_select_kernel(const float *poolq, const float *poolk, const float *poolv, float *scores_out, int *indices,
@@ -143,8 +154,8 @@ score_select_kernel(const float *poolq, const float *poolk, const float *poolv, 
     extern __shared__ __align__(16) float sm[];
     const int stride = score_stride(tiles);
     float *row_scores = sm;                                // [QT][stride]
-    float *stage = row_scores + (size_t)QT * stride;       // [KCHUNK][KPAD], later [VCHUNK][VD]
-    float *qrows = stage + KCHUNK * KPAD;                  // [QT][QPAD]
+    float *stage = row_scores + (size_t)QT * stride;       // [KCHUNK][KPART] (see staged()), later [VCHUNK][VD]
+    float *qrows = stage + KCHUNK * KPART;                 // [QT][QPAD]
 
     const int head = blockIdx.y, qt0 = blockIdx.x * QT;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -186,17 +197,17 @@ score_select_kernel(const float *poolq, const float *poolk, const float *poolv, 
 #pragma unroll
                 for (int u = 0; u < PER_THREAD; u++) {
                     const int i = tid + u * 256;
-                    *reinterpret_cast<float4 *>(stage + (i / (KPART / 4)) * KPAD + (i % (KPART / 4)) * 4) = next[u];
+                    *reinterpret_cast<float4 *>(stage + staged(i / (KPART / 4), i % (KPART / 4) * 4)) = next[u];
                 }
                 __syncthreads();
                 if (part + 1 < VD / KPART) fetch(k0, part + 1);
                 else if (k0 + KCHUNK < tiles) fetch(k0 + KCHUNK, 0);
                 if (!busy) continue;
-#pragma unroll 2
+#pragma unroll
                 for (int d = 0; d < KPART; d += 4) {
                     float4 kv[4], qv[NQ];
 #pragma unroll
-                    for (int i = 0; i < 4; i++) kv[i] = *reinterpret_cast<const float4 *>(stage + (key0 + 8 * i) * KPAD + d);
+                    for (int i = 0; i < 4; i++) kv[i] = *reinterpret_cast<const float4 *>(stage + staged(key0, d) + 8 * i * KPART);
 #pragma unroll
                     for (int u = 0; u < NQ; u++)
                         qv[u] = *reinterpret_cast<const float4 *>(qrows + (q0 + 4 * u) * QPAD + part * KPART + d);
@@ -463,10 +474,6 @@ cudaError_t vsa_tile_pool3(const void *const src[3], void *const tiled[3], float
                              tiles, heads);
 }
 
-static size_t score_select_smem(int tiles, int qt) {
-    return sizeof(float) * ((size_t)qt * score_stride(tiles) + KCHUNK * KPAD + (size_t)qt * QPAD);
-}
-
 template <int QPW>
 static cudaError_t launch_score_select(const float *poolq, const float *poolk, const float *poolv,
                                        float *scores, int *indices, int *counts, float *compression,
@@ -494,7 +501,7 @@ cudaError_t vsa_score_select_compress(const float *poolq, const float *poolk, co
                                       int heads, float scale, cudaStream_t stream) {
     if (tiles < 1 || tiles > 4096 || keep < 1 || prefix < 0 || prefix > tiles)
         return cudaErrorInvalidValue;
-    // 16 query tiles per CTA up to 1400 tiles (two such CTAs share an SM up to about 1090 tiles,
+    // 16 query tiles per CTA up to 1400 tiles (two such CTAs share an SM up to 1152 tiles,
     // one beyond), 8 per CTA beyond that: the score rows of a CTA must fit its shared memory.
     // A CTA's time is its own chain of chunks (products bound by shared-memory wavefronts, a dozen counts per query
     // tile for the threshold), so a call takes about one CTA's time as long as every CTA is resident: with few
