@@ -1,4 +1,5 @@
 """Shared fixtures. GPU tests are marked `gpu`; everything else runs on CPU."""
+import ctypes as C
 import sys
 from pathlib import Path
 
@@ -35,6 +36,39 @@ def gpu(package):
     context = native.Native()
     yield context
     context.close()
+
+
+class Busy:
+    """An ordinary call of several milliseconds. What is queued behind it on the context's stream is pending before any of
+    it starts, so that kernels which may overlap do."""
+
+    def __init__(self, gpu):
+        from h3_omni_b200 import native
+        self.gpu, self.rows, self.heads, self.runtime = gpu, 24000, 24, native._cudart()
+        self.tensors = [gpu.empty_bf16(self.rows * self.heads * 128) for _ in range(2)]
+        gpu.call("zero", self.tensors[1])
+        self.event = C.c_void_p()
+        assert self.runtime.cudaEventCreate(C.byref(self.event)) == 0
+
+    def queue(self):
+        out, x = self.tensors
+        self.gpu.call("sdpa_bf16", out, x, x, x, self.rows, self.heads, 128, 0.0883883476)
+        assert self.runtime.cudaEventRecord(self.event, C.c_void_p(self.gpu.lib.h3b_gpu_stream(self.gpu.gpu))) == 0
+
+    def running(self):
+        return self.runtime.cudaEventQuery(self.event) == 600   # cudaErrorNotReady
+
+    def close(self):
+        self.runtime.cudaEventDestroy(self.event)
+        for t in self.tensors:
+            self.gpu.free(t)
+
+
+@pytest.fixture(scope="session")
+def busy(gpu):
+    b = Busy(gpu)
+    yield b
+    b.close()
 
 
 def metrics(got, want):

@@ -351,9 +351,10 @@ def test_causal_rows_see_nothing_of_later_values(gpu, oracle, L, key):
 
 @pytest.mark.parametrize("kind,L", [("sdpa_bf16", 77), ("sdpa_bf16", 300), ("gqa_causal_bf16", 300), ("sdpa_f16_d64", 300),
                                     ("cross_attention_bf16", 5000)])
-def test_calls_that_overlap_see_each_other(gpu, oracle, kind, L):
+def test_calls_that_overlap_see_each_other(gpu, oracle, busy, kind, L):
     """A kernel may be set up while the one before it runs. Calls that read what the call before wrote and write what it
-    read (query and output change places) give the bits of the same calls waited for one by one."""
+    read (query and output change places), all pending before the first of them starts, give the bits of the same calls
+    waited for one by one."""
     from h3_omni_b200 import native
     f16, H = kind == "sdpa_f16_d64", 4
     rows, dtype = (64 if kind == "cross_attention_bf16" else L), native.F16 if f16 else native.BF16
@@ -363,6 +364,8 @@ def test_calls_that_overlap_see_each_other(gpu, oracle, kind, L):
     got = []
     for wait in (True, False):
         a, b, tk, tv = (gpu.tensor(x, dtype) for x in (q, q, k, v))
+        if not wait:
+            busy.queue()
         for _ in range(12):
             if kind == "cross_attention_bf16":
                 gpu.call(kind, b, 0, a, 0, tk, tv, 0, rows, L, H)
@@ -373,6 +376,7 @@ def test_calls_that_overlap_see_each_other(gpu, oracle, kind, L):
             a, b = b, a
             if wait:
                 gpu.submit()
+        assert wait or busy.running()
         got.append(gpu.read(a, q.shape))
     assert np.array_equal(*got)
     assert gpu.device_status() == 0
