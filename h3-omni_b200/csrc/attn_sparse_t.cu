@@ -57,20 +57,6 @@ constexpr int ST_S_COL = 0, ST_O_COL = 128;   // TMEM: S^T[2] at 0 / 64, O^T[2] 
 constexpr int ST_TMEM_COLS = 256;
 constexpr int ENC_NEG_INF = (int)0x807fffffu;   // encode(-inf)
 
-#ifdef H3B_TRACE
-// Development aid, compiled only with -DH3B_TRACE: cycle counters of CTA 0.
-__device__ long long g_sparse_trace[64];
-#define TR_DECL long long tr_acc[8] = {}; const long long tr_begin = clock64()
-#define TR_T0 const long long tr_t0 = clock64()
-#define TR_ADD(slot) tr_acc[slot] += clock64() - tr_t0
-#define TR_OUT(base, n) if (blockIdx.x == 0) { g_sparse_trace[base] = clock64() - tr_begin; for (int x = 0; x < n; x++) g_sparse_trace[base + 1 + x] = tr_acc[x]; }
-#else
-#define TR_DECL
-#define TR_T0
-#define TR_ADD(slot)
-#define TR_OUT(base, n)
-#endif
-
 struct SparseTParams {
     const int *indices, *counts, *sizes;
     __nv_bfloat16 *out;
@@ -296,7 +282,6 @@ attn_sparse_t_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
             tma_prefetch_desc(&map_q);
             tma_prefetch_desc(&map_k);
             tma_prefetch_desc(&map_v);
-            TR_DECL;
             struct Cursor {
                 Item it;
                 int item, j, g;
@@ -361,7 +346,6 @@ attn_sparse_t_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
                     }
                 }
             }
-            TR_OUT(0, 1);
         } else if (warp == 9) {
             // ------------------------------ QK issue: S^T[g & 1] = K pair . Q^T ------------------------------
             // The whole warp walks the loop and one elected lane issues: inside a one-lane branch
@@ -374,7 +358,6 @@ attn_sparse_t_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
             const uint32_t q_lo0 = (uint32_t)q_proto, q_hi = (uint32_t)(q_proto >> 32);
             const uint32_t k_lo0 = (uint32_t)k_proto, k_hi = (uint32_t)(k_proto >> 32);
             int g = 0, q_uses0 = 0, q_uses1 = 0;
-            TR_DECL;
             for (int i = 0;; i++) {
                 Item it;
                 if (!fetch_warp(i, it) || it.n < 0) break;
@@ -387,15 +370,10 @@ attn_sparse_t_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
                 bool ok = true;
                 for (int j = 0; j < it.n; j++, g++) {
                     const int slot = g & 1;
-                    {
-                        TR_T0;
-                        ok = mbar_wait_converged(bar_k_full(slot), (g >> 1) & 1, &abort_word) &&
-                             // the softmax group has finished reading S^T of step g - 2
-                             (g < 2 || mbar_wait_converged(bar_p_full(slot), ((g - 2) >> 1) & 1, &abort_word));
-                        TR_ADD(0);
-                    }
+                    ok = mbar_wait_converged(bar_k_full(slot), (g >> 1) & 1, &abort_word) &&
+                         // the softmax group has finished reading S^T of step g - 2
+                         (g < 2 || mbar_wait_converged(bar_p_full(slot), ((g - 2) >> 1) & 1, &abort_word));
                     if (!ok) break;
-                    TR_T0;
                     tc5_fence_after();
                     const uint32_t a_lo = k_lo0 + slot * (ST_SLOT >> 4), d_tmem = tmem + ST_S_COL + slot * 64;
                     if (leader) {
@@ -407,14 +385,9 @@ attn_sparse_t_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
                         mma_commit(bar_k_empty(slot));
                     }
                     __syncwarp();
-                    TR_ADD(1);
                 }
                 if (!ok) break;
             }
-#ifdef H3B_TRACE
-            tr_acc[2] = g;
-#endif
-            if (lane == 0) TR_OUT(8, 3);
         } else if (warp == 11) {
             // ------------------------------ PV issue: O^T[item & 1] += V pair^T . P^T[g & 1] ------------------------------
             const bool leader = elect_one();
@@ -424,7 +397,6 @@ attn_sparse_t_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
             const uint32_t v_lo0 = (uint32_t)v_proto, v_hi = (uint32_t)(v_proto >> 32);
             const uint32_t p_lo0 = (uint32_t)p_proto, p_hi = (uint32_t)(p_proto >> 32);
             int g = 0;
-            TR_DECL;
             for (int i = 0;; i++) {
                 Item it;
                 const int b = i & 1;
@@ -440,14 +412,9 @@ attn_sparse_t_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
                 bool ok = true;
                 for (int j = 0; j < it.n; j++, g++) {
                     const int slot = g & 1;
-                    {
-                        TR_T0;
-                        ok = mbar_wait_converged(bar_v_full(slot), (g >> 1) & 1, &abort_word) &&
-                             mbar_wait_converged(bar_p_full(slot), (g >> 1) & 1, &abort_word);
-                        TR_ADD(0);
-                    }
+                    ok = mbar_wait_converged(bar_v_full(slot), (g >> 1) & 1, &abort_word) &&
+                         mbar_wait_converged(bar_p_full(slot), (g >> 1) & 1, &abort_word);
                     if (!ok) break;
-                    TR_T0;
                     tc5_fence_after();
                     const uint32_t a_lo = v_lo0 + slot * (ST_SLOT >> 4), b_lo = p_lo0 + slot * (ST_P >> 4);
                     if (leader) {
@@ -465,13 +432,11 @@ attn_sparse_t_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
                         mma_commit(bar_pv_done(slot));
                     }
                     __syncwarp();
-                    TR_ADD(1);
                 }
                 if (!ok) break;
                 if (leader) mma_commit(bar_item_done(b));
                 __syncwarp();
             }
-            if (lane == 0) TR_OUT(12, 2);
         }
     } else if (warp >= 12) {
         warpgroup_reg_dec<64>();
@@ -543,7 +508,6 @@ attn_sparse_t_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
         int G = 0;   // global number of the current item's first step
         int ref_uses0 = 0, ref_uses1 = 0;   // items with a list seen so far, per buffer
         bool alive = true;
-        TR_DECL;
         for (int i = 0; alive; i++) {
             const int b = i & 1;
             Item it;
@@ -552,13 +516,8 @@ attn_sparse_t_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
             bool have_ref = false;
             for (int j = (G & 1) == k ? 0 : 1; j < it.n; j += 2) {
                 const int g = G + j;
-                {
-                    TR_T0;
-                    alive = __all_sync(0xffffffffu, mbar_wait(bar_s_full(k), (g >> 1) & 1, &abort_word));
-                    TR_ADD(0);
-                }
+                alive = __all_sync(0xffffffffu, mbar_wait(bar_s_full(k), (g >> 1) & 1, &abort_word));
                 if (!alive) break;
-                TR_T0;
                 tc5_fence_after();
                 uint32_t s0[32], s1[32];
                 tmem_ld32(s_addr, s0);
@@ -604,10 +563,8 @@ attn_sparse_t_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
                 tc5_fence_before();
                 fence_async_smem();
                 mbar_arrive(bar_p_full(k));
-                TR_ADD(1);
             }
             if (!alive) break;
-            TR_T0;
             // ---- item end: this warp's row sums, reduced over its 32 key rows in a fixed order ----
             if (i >= 2) {
                 alive = __all_sync(0xffffffffu, mbar_wait(bar_item_free(b), ((i >> 1) - 1) & 1, &abort_word));
@@ -657,9 +614,7 @@ attn_sparse_t_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
             if (lane == 0) mbar_arrive(bar_item_done(b));
             G += it.n;
             if (it.n > 0) (b ? ref_uses1 : ref_uses0)++;
-            TR_ADD(2);
         }
-        if ((tid & 127) == 0) TR_OUT(16 + 8 * k, 3);
     }
 
     // ---------------------------------- teardown ----------------------------------
@@ -677,12 +632,6 @@ attn_sparse_t_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
 }
 
 }  // namespace
-
-#ifdef H3B_TRACE
-extern "C" cudaError_t h3b_debug_sparse_trace(long long *host64) {
-    return cudaMemcpyFromSymbol(host64, g_sparse_trace, sizeof(long long) * 64);
-}
-#endif
 
 cudaError_t attn_sparse_t_launch(const CUtensorMap_st *mq, const CUtensorMap_st *mk, const CUtensorMap_st *mv,
                                  void *out, float *lse, const int *indices, const int *counts, const int *sizes,

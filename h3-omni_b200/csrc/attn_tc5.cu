@@ -436,7 +436,7 @@ attn_tc5_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
             mbar_arrive(bar_p_full(sb));
         }
 
-        // -------- epilogue: O / l -> bf16, straight to global memory --------
+        // -------- epilogue: O / l -> bf16, to global memory (dense: through shared) --------
         if (alive && n_tiles > 0) {
             alive = __all_sync(0xffffffffu,
                                mbar_wait(bar_pv_done, (n_tiles - 1) & 1, &abort_word));

@@ -58,16 +58,6 @@ struct PairConfig {
     static constexpr int SMEM_BYTES = 2 * Q_TILE_BYTES + STAGES * TILE_BYTES + 1024;
 };
 
-#ifdef H3B_TRACE
-// Development aid, compiled only with -DH3B_TRACE: cycle counters of CTA (0,0,0).
-__device__ long long g_pair_trace[32];
-#define TRACE_T0() const long long trace_t0 = clock64()
-#define TRACE_ADD(slot) g_pair_trace_local[slot] += clock64() - trace_t0
-#else
-#define TRACE_T0()
-#define TRACE_ADD(slot)
-#endif
-
 constexpr int PAIR_MAX_SEGMENTS = 6;
 // K/V may be given as up to six separate row ranges (live mode: text, sink, two recent chunks,
 // current chunk ...) that are attended as if concatenated; every range has its own tensor maps
@@ -283,10 +273,6 @@ attn_tc5_pair_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
                 }
                 __syncwarp();
             };
-#ifdef H3B_TRACE
-            long long g_pair_trace_local[8] = {};
-            const long long trace_begin = clock64();
-#endif
             auto release = [&](int tile) {   // the slot may be refilled once the MMAs issued so far are done
                 if (leader) mma_commit(bar_empty(tile % ST));
             };
@@ -305,29 +291,17 @@ attn_tc5_pair_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
             for (int j = 0; alive && j < n_tiles; j++) {
                 const bool more = j + 1 < n_tiles;
                 if (EVEN || j < steps_a) {
-                    {
-                        // P of tile A, and (through the ring watcher) V of this step and K of the next
-                        TRACE_T0();
-                        if (!mbar_wait_converged(bar_p_full(0, 0), j & 1, &abort_word)) break;
-                        TRACE_ADD(0);
-                    }
+                    // P of tile A, and (through the ring watcher) V of this step and K of the next
+                    if (!mbar_wait_converged(bar_p_full(0, 0), j & 1, &abort_word)) break;
                     tc5_fence_after();
-                    {
-                        TRACE_T0();
-                        issue_pv(j, 0, 0);
-                        if (!mbar_wait_converged(bar_p_full(0, 1), j & 1, &abort_word)) break;
-                        tc5_fence_after();
-                        issue_pv(j, 0, 1);
-                        if (!mbar_wait_converged(bar_p_full(0, 2), j & 1, &abort_word)) break;
-                        tc5_fence_after();
-                        issue_pv(j, 0, 2);
-                        TRACE_ADD(4);
-                    }
-                    if (EVEN ? more : j + 1 < steps_a) {
-                        TRACE_T0();
-                        issue_qk(j + 1, 0);
-                        TRACE_ADD(5);
-                    }
+                    issue_pv(j, 0, 0);
+                    if (!mbar_wait_converged(bar_p_full(0, 1), j & 1, &abort_word)) break;
+                    tc5_fence_after();
+                    issue_pv(j, 0, 1);
+                    if (!mbar_wait_converged(bar_p_full(0, 2), j & 1, &abort_word)) break;
+                    tc5_fence_after();
+                    issue_pv(j, 0, 2);
+                    if (EVEN ? more : j + 1 < steps_a) issue_qk(j + 1, 0);
                 } else {
                     // tile A has passed its diagonal (its watcher is done): V of this step directly
                     const int v = 2 * j + 1;
@@ -335,13 +309,8 @@ attn_tc5_pair_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
                     tc5_fence_after();
                 }
                 if (EVEN || j < steps_b) {
-                    {
-                        TRACE_T0();
-                        if (!mbar_wait_converged(bar_p_full(1, 0), j & 1, &abort_word)) break;
-                        TRACE_ADD(3);
-                    }
+                    if (!mbar_wait_converged(bar_p_full(1, 0), j & 1, &abort_word)) break;
                     tc5_fence_after();
-                    TRACE_T0();
                     issue_pv(j, 1, 0);
                     if (!mbar_wait_converged(bar_p_full(1, 1), j & 1, &abort_word)) break;
                     tc5_fence_after();
@@ -349,14 +318,11 @@ attn_tc5_pair_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
                     if (!mbar_wait_converged(bar_p_full(1, 2), j & 1, &abort_word)) break;
                     tc5_fence_after();
                     issue_pv(j, 1, 2);
-                    TRACE_ADD(6);
                 }
                 release(2 * j + 1);
                 if (more) {
-                    TRACE_T0();
                     if (EVEN || j + 1 < steps_b) issue_qk(j + 1, 1);
                     release(2 * j + 2);
-                    TRACE_ADD(7);
                 } else if (leader) {
                     mma_commit(bar_pv_done);      // both accumulators are final
                 }
@@ -365,20 +331,6 @@ attn_tc5_pair_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
             };
             if (!CAUSAL && has_b) walk(std::true_type{});
             else walk(std::false_type{});
-#ifdef H3B_TRACE
-            if (blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0 && lane == 0) {
-                g_pair_trace[0] = clock64() - trace_begin;   // MMA thread: whole walk
-                g_pair_trace[1] = g_pair_trace_local[0];     // waiting for P of tile A
-                g_pair_trace[2] = 0;
-                g_pair_trace[3] = 0;
-                g_pair_trace[4] = g_pair_trace_local[3];     // waiting for P of tile B
-                g_pair_trace[5] = n_tiles;
-                g_pair_trace[6] = g_pair_trace_local[4];     // thread time inside issue_pv(A)
-                g_pair_trace[7] = g_pair_trace_local[5];     // thread time inside issue_qk(A)
-                g_pair_trace[24] = g_pair_trace_local[6];    // the same for tile B: both PV halves with the wait between them
-                g_pair_trace[25] = g_pair_trace_local[7];    // issue_qk(B) and the ring release
-            }
-#endif
         }
     } else if (warp == 10) {
         // ------------------------------- ring watcher -------------------------------
@@ -405,10 +357,6 @@ attn_tc5_pair_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
         const int steps = t ? steps_b : steps_a;
         float m_ref = -INFINITY, l = 0.0f;
         bool alive = true;
-#ifdef H3B_TRACE
-        long long g_pair_trace_local[8] = {};
-        const long long trace_begin = clock64();
-#endif
         // One step of this thread's row: scores from TMEM (the whole row in registers, one read pass),
         // P back over them in three pieces. MASKED: only the first nvalid scores count.
         auto softmax_step = [&](auto masked, int j, int nvalid) {
@@ -489,35 +437,18 @@ attn_tc5_pair_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
             }
             const int in_range = min(PBN, seg_rows(seg) - seg_tile * PBN);
             seg_tile++;
-            {
-                TRACE_T0();
-                alive = __all_sync(0xffffffffu, mbar_wait_parked(bar_s_full(t), j & 1, &abort_word));
-                TRACE_ADD(0);
-            }
+            alive = __all_sync(0xffffffffu, mbar_wait_parked(bar_s_full(t), j & 1, &abort_word));
             if (!alive) break;
             tc5_fence_after();
-#ifdef H3B_TRACE
-            const long long trace_work = clock64();
-#endif
             // keys up to the row's own, counted from the tile's first key: of the warp's first row
             const int causal_first = q_row0 + t * PBM + (warp & 3) * 32 + 1 - j * PBN;
             if (min(in_range, CAUSAL ? causal_first : PBN) >= PBN)
                 softmax_step(std::false_type{}, j, PBN);
             else
                 softmax_step(std::true_type{}, j, CAUSAL ? min(in_range, causal_first + lane) : in_range);
-#ifdef H3B_TRACE
-            g_pair_trace_local[1] += clock64() - trace_work;
-#endif
         }
-#ifdef H3B_TRACE
-        if (blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0 && (tid & 127) == 0) {
-            g_pair_trace[8 + 4 * t] = clock64() - trace_begin;       // softmax warpgroup t: whole walk
-            g_pair_trace[9 + 4 * t] = g_pair_trace_local[0];         // waiting for S
-            g_pair_trace[10 + 4 * t] = g_pair_trace_local[1];        // S ready -> P delivered
-        }
-#endif
 
-        // -------- epilogue: O / l -> bf16, straight to global memory --------
+        // -------- epilogue: O / l -> 16 bits, through shared memory to global --------
         alive = alive && steps > 0;
         if (alive) alive = __all_sync(0xffffffffu, mbar_wait(bar_pv_done, 0, &abort_word));
         if (alive) {
@@ -705,9 +636,3 @@ cudaError_t attn_dense_tc5_pair(const CUtensorMap_st *mq, const CUtensorMap_st *
 }
 
 }  // namespace h3b
-
-#ifdef H3B_TRACE
-extern "C" cudaError_t h3b_debug_pair_trace(long long *host32) {
-    return cudaMemcpyFromSymbol(host32, h3b::g_pair_trace, sizeof(long long) * 32);
-}
-#endif
